@@ -155,6 +155,7 @@ extern "C" void bm_ctx_destroy(bm_ctx* ctx) {
     bm_cuda_free(ctx->stage);
     bm_cuda_free(ctx->flush_buf);
     bm_cuda_free(ctx->tscr);
+    bm_cuda_free(ctx->pscr);
     bm_cuda_free(ctx->rwork); bm_cuda_free(ctx->spart); bm_cuda_free(ctx->scnt); bm_cuda_free(ctx->rpart); bm_cuda_free(ctx->slots);
     if (ctx->hstage) bm_cuda_host_free(ctx->hstage);
     if (ctx->h_slots) bm_cuda_host_free(ctx->h_slots);
@@ -288,6 +289,7 @@ extern "C" bm_status bm_set_graph(bm_ctx* ctx, int side, int32_t n, int64_t m, c
     G.max_deg = H.max_deg;
     G.max_wdeg = H.max_wdeg;
     G.has_self = H.has_self;
+    G.has_dup = H.has_dup;
     G.loaded = true;
     ctx->n = n;
     ctx->nvec = (n + 1 + 3) & ~3;

@@ -53,6 +53,7 @@ struct HostCsr {
     std::vector<unsigned long long> htab;
     int hlog2 = 0;
     int has_self = 0;
+    int has_dup = 0;     // some list names a neighbour more than once (A only: B keeps one entry per edge)
     int32_t max_deg = 0;
     int64_t max_wdeg = 0;
     int64_t m_out() const { return optr.empty() ? 0 : optr.back(); }
@@ -178,6 +179,11 @@ inline int bm_build_host_csr(bool side_b, int32_t n, int64_t m, const int32_t* s
             if (side_b) ipos_of[(size_t)e] = p;
         }
     }
+    for (int32_t v = 1; v <= n && !G.has_dup; v++)
+        for (int32_t k = 1; k < ocnt[(size_t)v]; k++) {
+            const size_t p = (size_t)G.optr[(size_t)v] + (size_t)k;
+            if (bm_eid(G.oent[p]) == bm_eid(G.oent[p - 1])) { G.has_dup = 1; break; }
+        }
     if (side_b) {
         G.otw.assign((size_t)G.m_out(), -1);
         G.itw.assign((size_t)G.m_in(), -1);

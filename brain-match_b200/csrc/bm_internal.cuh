@@ -59,6 +59,7 @@ struct DevGraph {
     int32_t max_deg = 0;
     int64_t max_wdeg = 0;
     int has_self = 0;
+    int has_dup = 0;     // A: some list names a neighbour more than once
     bool loaded = false;
 };
 
@@ -105,6 +106,8 @@ struct bm_ctx {
     size_t flush_bytes = 0;
     void* tscr = nullptr;           // scratch of the delta-table top-K
     size_t tscr_bytes = 0;
+    void* pscr = nullptr;           // scratch of grouped pair deltas (bm_pairs.cu), bounded
+    size_t pscr_bytes = 0;
     int64_t launches = 0;
     int32_t row_ctas = 0;           // CTAs per row (cluster size); 0 = auto
     int32_t row_threads = 512;
@@ -313,8 +316,10 @@ bm_status bm_launch_score(bm_ctx* ctx, int64_t* score_out);
 bm_status bm_check_score(bm_ctx* ctx);
 bm_status bm_launch_relabel(bm_ctx* ctx);
 // exact_only: score differences whatever the context's delta semantics (for
-// callers that apply swaps regardless of their deltas and track the score)
-bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_out, bool exact_only = false);
+// callers that apply swaps regardless of their deltas and track the score);
+// run: how many consecutive pairs are known to share their first vertex
+bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_out, bool exact_only = false,
+                          int64_t run = 1);
 // Allocate the split-row buffers for the current n and refresh the per-row
 // work estimate (after the mapping is set); refresh alone after many swaps.
 bm_status bm_rows_prepare(bm_ctx* ctx);

@@ -2374,7 +2374,7 @@ extern "C" bm_status bm_search_learned(bm_ctx* ctx, bm_mlp* M, const int32_t* ro
         if (!p->uniform && (s = check_flag(M)) != BM_OK) return s;
         ta = clk::now();
         const int64_t kk = (int64_t)k * K;
-        if ((s = bm_launch_pairs(ctx, d_p, kk, (int64_t*)d_d)) != BM_OK) return s;
+        if ((s = bm_launch_pairs(ctx, d_p, kk, (int64_t*)d_d, false, K)) != BM_OK) return s;
         BM_CUDA(ctx, cudaMemcpyAsync(h_p.data(), d_p, sizeof(int32_t) * 2 * (size_t)kk, cudaMemcpyDeviceToHost,
                                      ctx->stream));
         BM_CUDA(ctx, cudaMemcpyAsync(h_d.data(), d_d, sizeof(long long) * (size_t)kk, cudaMemcpyDeviceToHost,
