@@ -19,14 +19,28 @@
 // sum moves every member's external and internal edges as if the other end
 // stayed; the second repairs each internal edge to its true new value.
 //
-// One CTA per set: the B rows of the members' images (out and in, B ids,
-// sorted) are staged in shared memory, then the members' lists are scanned
-// once with k-1 lookups per entry, binary searches in the staged rows (the
-// hash for rows that do not fit), atomics into g in shared memory; then the
-// k! permutations are enumerated in lexicographic order, each thread a
-// contiguous block stepped by
-// the lexicographic successor (the permutation packed in one register), and
-// reduced to the best (largest delta, lowest index).
+// One CTA per set.  The B rows of the members' images (out and in) mark, in a
+// table indexed by the low bits of the id, which members' rows may hold it;
+// the members' lists are then scanned once, and only an entry that meets a
+// mark looks its weight up in the hash, atomics into g in shared memory.
+// (Binary searches of the k-1 rows, staged in shared memory, for every entry
+// took 146,000 of a set's cycles on average, this scan 53,000: what bounds it
+// now is the latency of the lookups of hubs, which are in most rows.)
+//
+// The best permutation (largest delta, the first in lexicographic order on
+// ties) is then found in one of two ways.  The delta is a sum of one term per
+// member but for the internal entries.  With the images of a vertex cover of
+// the internal entries fixed, every other member's term depends on its own
+// image alone, and those members form an assignment problem, solved by a table
+// over subsets of the images left: E[mask] = the best total of the members not
+// yet placed when the images of mask are taken, 2^m values for m members,
+// filled from the full mask down.  So the c members of a smallest cover are
+// enumerated, k!/(k-c)! choices, a warp to a choice.  A sparse graph's random
+// sets have c = 0 (one table of 256 values instead of 40,320 permutations at
+// k = 8) or, with a hub among them, c = 1.  Past the limit of cover_limit(),
+// for calls that want every permutation's delta, and for k < 6, the k!
+// permutations are enumerated, each thread a contiguous block stepped by the
+// lexicographic successor (the permutation packed in one register).
 #include <climits>
 #include <vector>
 
@@ -54,14 +68,17 @@ struct KsetArgs {
     int32_t* best_perm;  // nsets * k
     long long* all;      // nsets * kfact, optional
     int32_t* status;     // nonzero: some set was rejected (see bm_kset_eval)
-    // B's rows in B ids (sorted by id): the gains' lookups are staged from them
+    // B's rows in B ids
     const int32_t* Bout_ptr;
     const int32_t* Bin_ptr;
     const uint32_t* Bout_ent0;
     const uint32_t* Bin_ent0;
 };
 
-constexpr int kKsetRowCap = 8192;  // B-row entries a set stages in shared memory (the rest: hash)
+// Row marks per direction, indexed by the id's low bits: exact up to 16,384
+// ids; beyond, two ids that share a mark cost a lookup that finds nothing.
+constexpr int kMaskIds = 16384;
+constexpr size_t kKsetSmem = 2 * kMaskIds;
 
 __device__ __forceinline__ void decode_perm(int32_t p, int k, int32_t* s) {
     int32_t avail[kMaxK];
@@ -185,9 +202,183 @@ __device__ void enumerate_perms(const KsetArgs& a, int64_t set, int32_t p0, int3
     }
 }
 
-__global__ void __launch_bounds__(kKThreads) kset_kernel(KsetArgs a) {
-    extern __shared__ uint32_t rowbuf[];  // kKsetRowCap entries
-    __shared__ int32_t r_off[2 * kMaxK], r_len[2 * kMaxK];  // row 2q: B-out(f_q), 2q+1: B-in(f_q); off -1: not staged
+// The c-th choice of images for the members of `cover` (in member order, images
+// in lexicographic order of the choice), as 4-bit fields at the members'
+// places; `used` gets the images taken.
+__device__ __forceinline__ uint32_t decode_choice(int32_t c, int k, uint32_t cover, int32_t count, uint32_t& used) {
+    uint32_t S = 0;
+    used = 0;
+    int32_t radix = count;  // choices of the members from here on
+    int left = k;
+    for (uint32_t m = cover; m; m &= m - 1, left--) {
+        const int i = __ffs(m) - 1;
+        radix /= left;
+        int idx = c / radix;
+        c -= idx * radix;
+        uint32_t avail = ~used & ((1u << k) - 1u);
+        for (; idx > 0; idx--) avail &= avail - 1;
+        const uint32_t q = (uint32_t)__ffs(avail) - 1u;
+        S |= q << (4 * i);
+        used |= 1u << q;
+    }
+    return S;
+}
+
+constexpr int kCoverChoices = 336;  // 8 * 7 * 6: the most choices of a cover (see cover_limit)
+
+// The largest cover that is enumerated; -1: always the permutations.  A choice
+// costs a warp about 300 instructions, a permutation a thread about 100, so
+// k!/(k-c)! choices on 8 warps stay below k! permutations on 256 threads up to
+// c = 3 at k = 8 (336 choices against 40,320), 2 at k = 7 and 1 at k = 6.
+__device__ __forceinline__ int cover_limit(int k) { return k - 5 > 0 ? k - 5 : -1; }
+
+struct CoverSmem {
+    long long E[1024];                  // 256 values for c = 0, else 128 to a warp
+    int32_t W[kKThreads / 32][64];      // gains of the members left, by the images left
+    long long val[kCoverChoices];
+    unsigned key;
+    int cover;
+};
+
+// Change of an internal entry's term when its ends take images si and sj.
+__device__ __forceinline__ int32_t repair(int32_t w, const int32_t* Bsub, int k, int i, int j, int si, int sj) {
+    return imin(w, Bsub[si * k + sj]) + imin(w, Bsub[i * k + j]) - imin(w, Bsub[si * k + j]) - imin(w, Bsub[i * k + sj]);
+}
+
+// The place-th set bit of m.
+__device__ __forceinline__ int nth_bit(uint32_t m, int place) {
+    for (; place > 0; place--) m &= m - 1;
+    return __ffs(m) - 1;
+}
+
+// One choice of the cover's images (fields S, images `used`): the gains of the
+// members left in W, the table in E, by the threads t, t + STRIDE, ... of a
+// warp or the whole CTA; returns the choice's best total (E[0] and the cover's
+// own terms).
+template <int STRIDE>
+__device__ long long cover_choice(int k, const int32_t* g, const int32_t* Bsub, const int32_t* sA, const int32_t* sB,
+                                  int32_t ni, const int32_t* ie_i, const int32_t* ie_j, const int32_t* ie_w,
+                                  uint32_t cover, uint32_t S, uint32_t used, int t, int32_t* W, long long* E) {
+    const uint32_t full = (1u << k) - 1u, rest = full & ~cover, left = full & ~used;
+    const int m = __popc(rest);
+    auto sync = [] { if (STRIDE == 32) __syncwarp(); else __syncthreads(); };
+    sync();  // the last choice's tables are no longer read
+    for (int e = t; e < m * m; e += STRIDE) {
+        const int i = nth_bit(rest, e / m), q = nth_bit(left, e % m);
+        int32_t d = g[i * k + q] + imin(sA[i], sB[q]);
+        for (int32_t n = 0; n < ni; n++) {
+            const int x = ie_i[n], y = ie_j[n];
+            if (x == i) d += repair(ie_w[n], Bsub, k, x, y, q, (int)nib(S, y));
+            else if (y == i) d += repair(ie_w[n], Bsub, k, x, y, (int)nib(S, x), q);
+        }
+        W[e] = d;
+    }
+    if (t == 0) E[(1 << m) - 1] = 0;
+    sync();
+    for (int lev = m - 1; lev >= 0; lev--) {
+        for (int mask = t; mask < (1 << m) - 1; mask += STRIDE) {
+            if (__popc((unsigned)mask) != lev) continue;
+            long long best = LLONG_MIN;
+            for (uint32_t av = ((1u << m) - 1u) & ~(uint32_t)mask; av; av &= av - 1) {
+                const int q = __ffs(av) - 1;
+                const long long v = (long long)W[lev * m + q] + E[mask | (1 << q)];
+                if (v > best) best = v;
+            }
+            E[mask] = best;
+        }
+        sync();
+    }
+    long long v = E[0];
+    for (uint32_t c = cover; c; c &= c - 1) {
+        const int i = __ffs(c) - 1, q = (int)nib(S, i);
+        v += (long long)g[i * k + q] + imin(sA[i], sB[q]);
+    }
+    for (int32_t n = 0; n < ni; n++) {
+        const int x = ie_i[n], y = ie_j[n];
+        if (((cover >> x) & 1u) && ((cover >> y) & 1u))
+            v += repair(ie_w[n], Bsub, k, x, y, (int)nib(S, x), (int)nib(S, y));
+    }
+    return v;
+}
+
+// The first permutation in lexicographic order that completes a choice to its
+// best total, as a field string with member 0 foremost.
+__device__ uint32_t cover_key(int k, uint32_t cover, uint32_t S, uint32_t used, const int32_t* W, const long long* E) {
+    const uint32_t full = (1u << k) - 1u, left = full & ~used;
+    const int m = __popc(left);
+    uint32_t key = 0, mask = 0;
+    int lev = 0;
+    for (int i = 0; i < k; i++) {
+        int q = (int)nib(S, i);
+        if (!((cover >> i) & 1u)) {
+            int a = 0;
+            for (uint32_t av = ((1u << m) - 1u) & ~mask; av; av &= av - 1) {
+                a = __ffs(av) - 1;
+                if ((long long)W[lev * m + a] + E[mask | (1u << a)] == E[mask]) break;
+            }
+            mask |= 1u << a;
+            lev++;
+            q = nth_bit(left, a);
+        }
+        key |= (uint32_t)q << (28 - 4 * i);
+    }
+    return key;
+}
+
+// Best permutation of one set with the images of `cover` enumerated; whole
+// CTA.  sA is zero when there are no self-loop terms.
+__device__ void best_by_cover(const KsetArgs& a, int64_t set, const int32_t* g, const int32_t* Bsub, const int32_t* sA,
+                              const int32_t* sB, int32_t ni, const int32_t* ie_i, const int32_t* ie_j,
+                              const int32_t* ie_w, uint32_t cover, CoverSmem& cs) {
+    const int k = a.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c = __popc(cover);
+    if (tid == 0) cs.key = 0xFFFFFFFFu;
+    long long top;
+    if (c == 0) {
+        top = cover_choice<kKThreads>(k, g, Bsub, sA, sB, ni, ie_i, ie_j, ie_w, 0u, 0u, 0u, tid, cs.W[0], cs.E);
+        if (tid == 0) cs.key = cover_key(k, 0u, 0u, 0u, cs.W[0], cs.E);
+    } else {
+        int32_t count = 1;
+        for (int t = 0; t < c; t++) count *= k - t;
+        long long* E = cs.E + 128 * warp;
+        for (int32_t ch = warp; ch < count; ch += kKThreads / 32) {
+            uint32_t used;
+            const uint32_t S = decode_choice(ch, k, cover, count, used);
+            const long long v =
+                cover_choice<32>(k, g, Bsub, sA, sB, ni, ie_i, ie_j, ie_w, cover, S, used, lane, cs.W[warp], E);
+            if (lane == 0) cs.val[ch] = v;
+        }
+        __syncthreads();
+        top = LLONG_MIN;
+        for (int32_t ch = lane; ch < count; ch += 32) top = max(top, cs.val[ch]);
+        for (int o = 16; o; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+        for (int32_t ch = warp; ch < count; ch += kKThreads / 32) {
+            if (cs.val[ch] != top) continue;
+            uint32_t used;
+            const uint32_t S = decode_choice(ch, k, cover, count, used);
+            if (count > kKThreads / 32)  // else the warp's tables are still this choice's
+                cover_choice<32>(k, g, Bsub, sA, sB, ni, ie_i, ie_j, ie_w, cover, S, used, lane, cs.W[warp], E);
+            if (lane == 0) atomicMin(&cs.key, cover_key(k, cover, S, used, cs.W[warp], E));
+        }
+    }
+    __syncthreads();
+    if (tid < k) a.best_perm[set * k + tid] = (int32_t)((cs.key >> (28 - 4 * tid)) & 15u);
+    if (tid == 0) {
+        long long base = 0;
+        for (int i = 0; i < k; i++) base += (long long)g[i * k + i] + imin(sA[i], sB[i]);
+        a.best_delta[set] = top - base;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(kKThreads, 4) kset_kernel(KsetArgs a) {
+    extern __shared__ uint32_t rmask[];  // per id, the members whose B-out row holds it, then whose B-in row: bytes
+    __shared__ CoverSmem cs;
+    __shared__ uint32_t adj[kMaxK];  // members joined to member i by internal entries
+    // the B rows (2q: B-out(f_q), 2q+1: B-in(f_q)) and the A lists (2i: out(t_i),
+    // 2i+1: in(t_i)) as two streams of quads: running ends, and starts less the
+    // quads before
+    __shared__ int32_t r_beg[2 * kMaxK], r_end[2 * kMaxK], l_beg[2 * kMaxK], l_end[2 * kMaxK];
     __shared__ int32_t t[kMaxK], f[kMaxK], sA[kMaxK], sB[kMaxK];
     __shared__ int32_t g[kMaxK * kMaxK], Bsub[kMaxK * kMaxK];
     __shared__ int32_t n_int, bad;
@@ -196,7 +387,10 @@ __global__ void __launch_bounds__(kKThreads) kset_kernel(KsetArgs a) {
     __shared__ int32_t red_p[kKThreads / 32];
     const int k = a.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int64_t set = blockIdx.x; set < a.nsets; set += gridDim.x) {
-        if (tid == 0) { n_int = 0; bad = 0; }
+        if (tid == 0) n_int = bad = 0;
+        if (tid < kMaxK) adj[tid] = 0u;
+        for (int32_t i = tid; i < 2 * kMaskIds / 16; i += kKThreads)
+            reinterpret_cast<uint4*>(rmask)[i] = make_uint4(0u, 0u, 0u, 0u);
         if (tid < k) {
             const int32_t v = a.sets[set * k + tid];
             t[tid] = v;
@@ -204,10 +398,7 @@ __global__ void __launch_bounds__(kKThreads) kset_kernel(KsetArgs a) {
         }
         if (tid < k * k) g[tid] = 0;
         __syncthreads();
-        if (tid == 0)
-            for (int i = 0; i < k; i++)
-                for (int j = i + 1; j < k; j++)
-                    if (t[i] == t[j]) bad = 1;
+        if (tid < k * k && tid / k < tid % k && t[tid / k] == t[tid % k]) bad = 1;
         __syncthreads();
         if (bad) {
             if (tid < k) a.best_perm[set * k + tid] = tid;
@@ -227,55 +418,84 @@ __global__ void __launch_bounds__(kKThreads) kset_kernel(KsetArgs a) {
             const int p = tid / k, q = tid % k;
             Bsub[tid] = (p == q) ? 0 : bm_hash_get(a.hb, f[p], f[q]);
         }
-        // ---- stage the B rows of the members' images (out and in), in order,
-        // while they fit
-        if (tid == 0) {
-            int32_t off = 0;
-            for (int r = 0; r < 2 * k; r++) {
-                const int32_t* ptr = (r & 1) ? a.Bin_ptr : a.Bout_ptr;
-                const int32_t g0 = f[r >> 1];
-                const int32_t len = ptr[g0 + 1] - ptr[g0];
-                r_len[r] = len;
-                r_off[r] = (off + len <= kKsetRowCap) ? off : -1;
-                if (r_off[r] >= 0) off += len;
+        // ---- bounds of all rows and lists
+        if (tid < 4 * k) {
+            const bool row = tid < 2 * k;
+            const int l = row ? tid : tid - 2 * k;
+            const int32_t* ptr = row ? ((l & 1) ? a.Bin_ptr : a.Bout_ptr) : ((l & 1) ? a.A.in_ptr : a.A.out_ptr);
+            const int32_t v = row ? f[l >> 1] : t[l >> 1];
+            (row ? r_beg : l_beg)[l] = ptr[v] >> 2;
+            (row ? r_end : l_end)[l] = ptr[v + 1] >> 2;
+        }
+        __syncthreads();
+        if (tid == 0 || tid == 32) {
+            int32_t* beg = tid ? l_beg : r_beg;
+            int32_t* end = tid ? l_end : r_end;
+            int32_t sum = 0;
+            for (int l = 0; l < 2 * k; l++) {
+                const int32_t b = beg[l];
+                beg[l] = b - sum;
+                sum += end[l] - b;
+                end[l] = sum;
             }
         }
         __syncthreads();
-        for (int r = 0; r < 2 * k; r++) {
-            if (r_off[r] < 0) continue;
-            const int32_t* ptr = (r & 1) ? a.Bin_ptr : a.Bout_ptr;
-            const uint32_t* ent = ((r & 1) ? a.Bin_ent0 : a.Bout_ent0) + ptr[f[r >> 1]];
-            for (int32_t j = tid; j < r_len[r]; j += kKThreads) rowbuf[r_off[r] + j] = ent[j];
+        const int nl = 2 * k;
+        auto list_of = [nl](const int32_t* end, int32_t q) {  // the list that quad q of a stream falls in
+            int l = 0;
+#pragma unroll
+            for (int step = 8; step; step >>= 1)
+                if (l + step < nl && end[l + step - 1] <= q) l += step;
+            return l;
+        };
+        // ---- marks of the B rows
+        for (int32_t q = tid; q < r_end[nl - 1]; q += kKThreads) {
+            const int r = list_of(r_end, q), dir = r & 1;
+            const uint4 e4 = __ldg(reinterpret_cast<const uint4*>(dir ? a.Bin_ent0 : a.Bout_ent0) + r_beg[r] + q);
+            const uint32_t en4[4] = {e4.x, e4.y, e4.z, e4.w};
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                if (en4[c] == 0) continue;
+                const uint32_t at = dir * kMaskIds + ((uint32_t)bm_eid(en4[c]) & (kMaskIds - 1));
+                atomicOr(rmask + (at >> 2), 1u << (8 * (at & 3) + (r >> 1)));
+            }
         }
         __syncthreads();
-        // ---- gains and internal entries: scan each member's out- and in-list
-        for (int i = 0; i < k; i++) {
-            for (int dir = 0; dir < 2; dir++) {
-                const int32_t* ptr = dir ? a.A.in_ptr : a.A.out_ptr;
-                const uint32_t* ent = dir ? a.A.in_ent : a.A.out_ent;
-                const int32_t b = ptr[t[i]], e = ptr[t[i] + 1];
-                for (int32_t j = b + tid; j < e; j += kKThreads) {
-                    const uint32_t en = ent[j];
-                    if (en == 0) continue;
-                    const int32_t x = bm_eid(en), w = bm_ew(en);
-                    const int32_t gx = a.pi[x];
-                    if (dir == 0) {
-                        for (int q = 0; q < k; q++)
-                            if (t[q] == x) {
-                                const int32_t slot = atomicAdd(&n_int, 1);
-                                if (slot < kMaxInternal) { ie_i[slot] = i; ie_j[slot] = q; ie_w[slot] = w; }
-                            }
-                    }
-                    for (int q = 0; q < k; q++) {
-                        if (q == i) continue;
-                        // out: B(f_q, pi x) in B-out(f_q); in: B(pi x, f_q) in B-in(f_q)
-                        const int r = 2 * q + dir;
-                        const int32_t bw = r_off[r] >= 0 ? bm_row_weight(rowbuf + r_off[r], r_len[r], gx)
-                                           : (dir ? bm_hash_get(a.hb, gx, f[q]) : bm_hash_get(a.hb, f[q], gx));
-                        const int32_t c = imin(w, bw);
-                        if (c) atomicAdd(&g[i * k + q], c);
-                    }
+        // ---- gains and internal entries: a thread a quad at a time; the lookups
+        // of its four entries run in one loop, so that a warp's lanes do theirs
+        // together
+        for (int32_t q = tid; q < l_end[nl - 1]; q += kKThreads) {
+            const int l = list_of(l_end, q), i = l >> 1, dir = l & 1;
+            const uint4 e4 = __ldg(reinterpret_cast<const uint4*>(dir ? a.A.in_ent : a.A.out_ent) + l_beg[l] + q);
+            const uint32_t en4[4] = {e4.x, e4.y, e4.z, e4.w};
+            int32_t gx4[4];
+            uint32_t found = 0;  // byte c: the rows that entry c meets
+#pragma unroll
+            for (int c = 0; c < 4; c++) gx4[c] = __ldg(a.pi + bm_eid(en4[c]));
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                const uint32_t m = reinterpret_cast<const uint8_t*>(rmask)[dir * kMaskIds + (gx4[c] & (kMaskIds - 1))];
+                found |= (en4[c] ? m & ~(1u << i) : 0u) << (8 * c);
+            }
+            if (dir == 0)
+                for (int m = 0; m < k; m++) {
+                    const uint32_t tm = (uint32_t)t[m];
+#pragma unroll
+                    for (int c = 0; c < 4; c++)
+                        if ((en4[c] & BM_ID_MASK) == tm) {
+                            const int32_t slot = atomicAdd(&n_int, 1);
+                            if (slot < kMaxInternal) { ie_i[slot] = i; ie_j[slot] = m; ie_w[slot] = bm_ew(en4[c]); }
+                            atomicOr(&adj[i], 1u << m);
+                            atomicOr(&adj[m], 1u << i);
+                        }
                 }
+            for (; found; found &= found - 1) {
+                const int b = __ffs(found) - 1, c = b >> 3, m = b & 7;
+                const int32_t gx = c == 0 ? gx4[0] : c == 1 ? gx4[1] : c == 2 ? gx4[2] : gx4[3];
+                const uint32_t en = c == 0 ? en4[0] : c == 1 ? en4[1] : c == 2 ? en4[2] : en4[3];
+                // out: B(f_m, pi x); in: B(pi x, f_m)
+                const int32_t d = imin(bm_ew(en), dir ? bm_hash_get(a.hb, gx, f[m]) : bm_hash_get(a.hb, f[m], gx));
+                if (d) atomicAdd(&g[i * k + m], d);
             }
         }
         __syncthreads();
@@ -283,6 +503,22 @@ __global__ void __launch_bounds__(kKThreads) kset_kernel(KsetArgs a) {
         if (tid == 0 && n_int > kMaxInternal) { bad = 1; atomicOr(a.status, 2); }
         __syncthreads();
         const int32_t ni = bad ? 0 : n_int;
+        const int climit = cover_limit(k);
+        if (climit >= 0 && !a.all && !bad) {
+            // the smallest vertex cover (the lowest mask on ties): a thread a mask
+            if (tid == 0) cs.cover = 0x7FFFFFFF;
+            __syncthreads();
+            if (tid < (1 << k)) {
+                bool covers = true;
+                for (int i = 0; i < k; i++) covers &= ((tid >> i) & 1) || (adj[i] & ~(uint32_t)tid) == 0u;
+                if (covers) atomicMin(&cs.cover, (__popc((unsigned)tid) << kMaxK) | tid);
+            }
+            __syncthreads();
+            if ((cs.cover >> kMaxK) <= climit) {
+                best_by_cover(a, set, g, Bsub, sA, sB, ni, ie_i, ie_j, ie_w, (uint32_t)cs.cover & ((1u << kMaxK) - 1u), cs);
+                continue;
+            }
+        }
         // ---- enumerate permutations
         int32_t per = (a.kfact + kKThreads - 1) / kKThreads;
         if (k >= 4) per = (per + 5) / 6 * 6;  // whole groups of six (see enumerate_perms)
@@ -438,8 +674,13 @@ bm_status bm_launch_kset(bm_ctx* ctx, int32_t k, const int32_t* d_sets, int64_t 
     a.best_perm = d_perm;
     a.all = d_all;
     a.status = d_status;
-    int64_t blocks = nsets < (int64_t)ctx->num_sms * 8 ? nsets : (int64_t)ctx->num_sms * 8;
-    kset_kernel<<<(unsigned)blocks, kKThreads, sizeof(uint32_t) * kKsetRowCap, ctx->stream>>>(a);
+    // a block per set: sets differ widely in cost (hubs, covers), and the
+    // hardware hands out blocks as they finish
+    const int64_t blocks = nsets < (1 << 20) ? nsets : (1 << 20);
+    BM_CUDA(ctx, cudaFuncSetAttribute(kset_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKsetSmem));
+    BM_CUDA(ctx, cudaFuncSetAttribute(kset_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                      (int)cudaSharedmemCarveoutMaxShared));
+    kset_kernel<<<(unsigned)blocks, kKThreads, kKsetSmem, ctx->stream>>>(a);
     BM_LAUNCH_CHECK(ctx, "kset_kernel");
     return BM_OK;
 }
