@@ -232,6 +232,22 @@ static bm_status upload(bm_ctx* ctx, T** d, const T* h, size_t count) {
         if (_s != BM_OK) return _s;        \
     } while (0)
 
+// Edge lists of at least this many entries are laid out on the device, smaller
+// ones by the host builder: 8,000 edges on 2,000 vertices take 0.70 (A) and
+// 0.54 ms (B) on the host, 8,300 take 0.51 and 0.43 ms on the device, whose
+// two dozen launches and allocations cost the same for any list.
+constexpr int64_t kDeviceBuildMin = 8192;
+
+// The new graph of a side takes the place of the old one, whose mapping goes.
+static void adopt_graph(bm_ctx* ctx, int side, const DevGraph& built) {
+    ctx->mapped = false;
+    free_graph(ctx->g[side]);
+    ctx->g[side] = built;
+    ctx->g[side].loaded = true;
+    ctx->n = built.n;
+    ctx->nvec = (built.n + 1 + 3) & ~3;
+}
+
 extern "C" bm_status bm_set_graph(bm_ctx* ctx, int side, int32_t n, int64_t m, const int32_t* src,
                                   const int32_t* dst, const int32_t* w) {
     if (!ctx) return BM_INVALID_ARG;
@@ -239,6 +255,22 @@ extern "C" bm_status bm_set_graph(bm_ctx* ctx, int side, int32_t n, int64_t m, c
     int other = 1 - side;
     if (ctx->g[other].loaded && ctx->g[other].n != n)
         return bm_fail(ctx, BM_INVALID_ARG, "n=%d differs from the other graph's n=%d", n, ctx->g[other].n);
+    if (n >= 1 && n <= BM_MAX_N && m >= kDeviceBuildMin && m < (int64_t)0x7fffffff - 4 * (int64_t)BM_MAX_N && src && dst && w) {
+        BM_CUDA(ctx, cudaSetDevice(ctx->device));
+        BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        DevGraph built;
+        bool rejected = false;
+        const bm_status st = bm_build_graph_dev(ctx, side == BM_SIDE_B, n, m, src, dst, w, built, &rejected);
+        if (st == BM_OK && !rejected) {
+            adopt_graph(ctx, side, built);
+            return BM_OK;
+        }
+        free_graph(built);
+        // a rejected input is worded by the host builder; without room for the
+        // old and the new graph together, it frees the old one first
+        if (st != BM_OK && st != BM_OOM) return st;
+        cudaGetLastError();
+    }
     HostCsr H;
     std::string err;
     if (bm_build_host_csr(side == BM_SIDE_B, n, m, src, dst, w, H, err) != 0)

@@ -217,15 +217,60 @@ __global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const int4* __re
     }
 }
 
-// Plain CSR (ids only) of one direction of an edge list, on the host.
-void build_adj(int32_t n, int64_t m, const int32_t* from, const int32_t* to, std::vector<int32_t>& ptr,
-               std::vector<int32_t>& idx) {
-    ptr.assign((size_t)n + 2, 0);
-    for (int64_t e = 0; e < m; e++) ptr[(size_t)from[e] + 1]++;
-    for (int32_t i = 1; i <= n + 1; i++) ptr[(size_t)i] += ptr[(size_t)i - 1];
-    idx.resize((size_t)std::max<int64_t>(m, 1));
-    std::vector<int32_t> fill(ptr.begin(), ptr.end() - 1);
-    for (int64_t e = 0; e < m; e++) idx[(size_t)fill[(size_t)from[e]]++] = to[e];
+// Plain adjacency (ids only, any order within a list: the features are counts)
+// of both directions of an edge list.
+__global__ void adj_count_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int32_t n,
+                                 int32_t* __restrict__ ocnt, int32_t* __restrict__ icnt, int* __restrict__ bad) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = src[e], d = dst[e];
+        if ((uint32_t)(s - 1) >= (uint32_t)n || (uint32_t)(d - 1) >= (uint32_t)n) {
+            *bad = 1;
+            continue;
+        }
+        atomicAdd(ocnt + s, 1);
+        atomicAdd(icnt + d, 1);
+    }
+}
+
+// Exclusive sums of the counts of one direction (block 0: out, 1: in) into
+// ptr[0..n+1] and the fill cursors.
+__global__ void __launch_bounds__(1024) adj_scan_kernel(int32_t* cnt0, int32_t* cnt1, int32_t n, int32_t* ptr0, int32_t* ptr1) {
+    __shared__ int32_t wsum[32];
+    int32_t* cnt = blockIdx.x ? cnt1 : cnt0;
+    int32_t* ptr = blockIdx.x ? ptr1 : ptr0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int32_t base = 0;
+    for (int32_t v0 = 0; v0 <= n; v0 += 1024) {
+        const int32_t v = v0 + tid, c = v <= n ? cnt[v] : 0;
+        int32_t s = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        if (lane == 31) wsum[warp] = s;
+        __syncthreads();
+        int32_t before = base;
+        for (int w = 0; w < 32; w++) {
+            if (w < warp) before += wsum[w];
+            base += wsum[w];
+        }
+        if (v <= n) {
+            ptr[v] = before + s - c;
+            cnt[v] = before + s - c;  // becomes the fill cursor
+        }
+        __syncthreads();
+    }
+    if (tid == 0) ptr[n + 1] = base;
+}
+
+__global__ void adj_fill_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m,
+                                int32_t* __restrict__ ocur, int32_t* __restrict__ icur, int32_t* __restrict__ oidx,
+                                int32_t* __restrict__ iidx) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
+        const int32_t s = src[e], d = dst[e];
+        oidx[atomicAdd(ocur + s, 1)] = d;
+        iidx[atomicAdd(icur + d, 1)] = s;
+    }
 }
 
 struct DevBuf {
@@ -244,23 +289,36 @@ struct DevBuf {
     }
 };
 
-// Features (n+1 int4: in, out, reach2, canreach2) of one graph on the device.
+// Features (n+1 int4: in, out, reach2, canreach2) of one graph on the device;
+// *bad is set when an endpoint lies outside 1..n.
 bm_status graph_features(bm_ctx* ctx, DevBuf& mem, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
-                         std::vector<int4>& feat) {
-    std::vector<int32_t> optr, oidx, iptr, iidx;
-    build_adj(n, m, src, dst, optr, oidx);
-    build_adj(n, m, dst, src, iptr, iidx);
-    int32_t *d_optr, *d_oidx, *d_iptr, *d_iidx;
+                         std::vector<int4>& feat, bool* bad) {
+    const size_t M = (size_t)m, V = (size_t)n + 2;
+    int32_t *d_src, *d_dst, *d_optr, *d_oidx, *d_iptr, *d_iidx, *d_cnt;
     int* d_next;
     int4* d_feat;
-    if (!mem.get(&d_optr, optr.size()) || !mem.get(&d_oidx, oidx.size()) || !mem.get(&d_iptr, iptr.size()) ||
-        !mem.get(&d_iidx, iidx.size()) || !mem.get(&d_next, 1) || !mem.get(&d_feat, (size_t)n + 1))
+    if (!mem.get(&d_src, M) || !mem.get(&d_dst, M) || !mem.get(&d_cnt, 2 * V) || !mem.get(&d_optr, V) ||
+        !mem.get(&d_oidx, M) || !mem.get(&d_iptr, V) || !mem.get(&d_iidx, M) || !mem.get(&d_next, 2) ||
+        !mem.get(&d_feat, (size_t)n + 1))
         return bm_fail(ctx, BM_OOM, "greedy matching: device allocation failed");
-    BM_CUDA(ctx, cudaMemcpyAsync(d_optr, optr.data(), sizeof(int32_t) * optr.size(), cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_oidx, oidx.data(), sizeof(int32_t) * oidx.size(), cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_iptr, iptr.data(), sizeof(int32_t) * iptr.size(), cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_iidx, iidx.data(), sizeof(int32_t) * iidx.size(), cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemsetAsync(d_next, 0, sizeof(int), ctx->stream));
+    if (m > 0) {
+        BM_CUDA(ctx, cudaMemcpyAsync(d_src, src, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
+        BM_CUDA(ctx, cudaMemcpyAsync(d_dst, dst, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    BM_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, sizeof(int32_t) * 2 * V, ctx->stream));
+    BM_CUDA(ctx, cudaMemsetAsync(d_next, 0, 2 * sizeof(int), ctx->stream));
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m + 255) / 256, (int64_t)ctx->num_sms * 8));
+    adj_count_kernel<<<grid, 256, 0, ctx->stream>>>(d_src, d_dst, m, n, d_cnt, d_cnt + V, d_next + 1);
+    BM_LAUNCH_CHECK(ctx, "adj_count_kernel");
+    int h_bad = 0;
+    BM_CUDA(ctx, cudaMemcpyAsync(&h_bad, d_next + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    *bad = h_bad != 0;
+    if (*bad) return BM_OK;
+    adj_scan_kernel<<<2, 1024, 0, ctx->stream>>>(d_cnt, d_cnt + V, n, d_optr, d_iptr);
+    BM_LAUNCH_CHECK(ctx, "adj_scan_kernel");
+    adj_fill_kernel<<<grid, 256, 0, ctx->stream>>>(d_src, d_dst, m, d_cnt, d_cnt + V, d_oidx, d_iidx);
+    BM_LAUNCH_CHECK(ctx, "adj_fill_kernel");
     BM_CUDA(ctx, cudaMemsetAsync(d_feat, 0, sizeof(int4) * ((size_t)n + 1), ctx->stream));
     const size_t smem = sizeof(uint32_t) * (((size_t)n + 32) / 32);
     if (smem > 48 * 1024)
@@ -284,18 +342,21 @@ extern "C" bm_status bm_greedy_match_dev(bm_ctx* ctx, int32_t n, int64_t mA, con
     if (mA < 0 || mB < 0 || mA >= INT32_MAX || mB >= INT32_MAX || (mA > 0 && (!srcA || !dstA)) ||
         (mB > 0 && (!srcB || !dstB)))
         return bm_fail(ctx, BM_INVALID_ARG, "bad edge arrays");
-    const int32_t* ends[4] = {srcA, dstA, srcB, dstB};
-    const int64_t ms[4] = {mA, mA, mB, mB};
-    for (int q = 0; q < 4; q++)
-        for (int64_t e = 0; e < ms[q]; e++)
-            if (ends[q][e] < 1 || ends[q][e] > n)
-                return bm_fail(ctx, BM_INVALID_ARG, "edge endpoint %d outside 1..%d", ends[q][e], n);
     BM_CUDA(ctx, cudaSetDevice(ctx->device));
     DevBuf mem;
     std::vector<int4> fa, fb;
     bm_status s;
-    if ((s = graph_features(ctx, mem, n, mA, srcA, dstA, fa)) != BM_OK) return s;
-    if ((s = graph_features(ctx, mem, n, mB, srcB, dstB, fb)) != BM_OK) return s;
+    bool badA = false, badB = false;
+    if ((s = graph_features(ctx, mem, n, mA, srcA, dstA, fa, &badA)) != BM_OK) return s;
+    if (!badA && (s = graph_features(ctx, mem, n, mB, srcB, dstB, fb, &badB)) != BM_OK) return s;
+    if (badA || badB) {
+        const int32_t* ends[4] = {srcA, dstA, srcB, dstB};
+        const int64_t ms[4] = {mA, mA, mB, mB};
+        for (int q = 0; q < 4; q++)
+            for (int64_t e = 0; e < ms[q]; e++)
+                if (ends[q][e] < 1 || ends[q][e] > n)
+                    return bm_fail(ctx, BM_INVALID_ARG, "edge endpoint %d outside 1..%d", ends[q][e], n);
+    }
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // both graphs' vertices by descending feature sum, ties by id
     auto order = [&](const std::vector<int4>& f, std::vector<int32_t>& ids, std::vector<int4>& sorted) {

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <algorithm>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -76,6 +77,26 @@ struct HashView {
     const unsigned long long* tab;
     int32_t log2;
     int32_t np1;  // n+1, key = g*(n+1)+h
+};
+
+// A host array that is sized without being written (a std::vector would touch
+// every page once before the copy from the device touches it again).
+template <typename T>
+struct HostArray {
+    std::unique_ptr<T[]> p;
+    size_t n = 0, cap = 0;
+    void resize(size_t count) {
+        if (count > cap) { p.reset(new T[count]); cap = count; }
+        n = count;
+    }
+    T* data() { return p.get(); }
+    size_t size() const { return n; }
+    const T& operator[](size_t i) const { return p[i]; }
+    HostArray& operator=(const std::vector<T>& v) {
+        resize(v.size());
+        std::copy(v.begin(), v.end(), p.get());
+        return *this;
+    }
 };
 
 struct bm_ctx {
@@ -148,7 +169,7 @@ struct bm_ctx {
     bool row_host_res = false;
     // host copy of A's adjacency (independence tests of batched swaps)
     std::vector<int32_t> hA_optr, hA_iptr;
-    std::vector<uint32_t> hA_oent, hA_ient;
+    HostArray<uint32_t> hA_oent, hA_ient;
     // device address of the allocation-free chain entry point's static
     // scratch on this context's device (bm_noalloc_setup, at creation)
     unsigned char* noalloc_scratch = nullptr;
@@ -315,6 +336,12 @@ bm_status bm_launch_score(bm_ctx* ctx, int64_t* score_out);
 // deltas) against it; the recomputed score is kept either way.
 bm_status bm_check_score(bm_ctx* ctx);
 bm_status bm_launch_relabel(bm_ctx* ctx);
+// Id-sorted lists oent, ient copied to out, in in bank-spread order of their
+// ids; tmp holds as many int32 as the longer of the two.
+bm_status bm_launch_spread(bm_ctx* ctx, int32_t n, const int32_t* optr, const int32_t* iptr, const uint32_t* oent,
+                           const uint32_t* ient, uint32_t* out, uint32_t* in, int32_t* tmp);
+bm_status bm_build_graph_dev(bm_ctx* ctx, bool side_b, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
+                             const int32_t* w, DevGraph& G, bool* rejected);
 // exact_only: score differences whatever the context's delta semantics (for
 // callers that apply swaps regardless of their deltas and track the score);
 // run: how many consecutive pairs are known to share their first vertex

@@ -90,6 +90,9 @@ score_kernel(GView A, HashView hb, const int32_t* __restrict__ selfB, const int3
 // banks not yet empty as one ballot.  A thread per list took 2.4 ms a launch
 // at full scale (a hub's 8,000 entries in one thread); both directions take
 // 0.75 ms so.
+//
+// Without pinv the ids stay as they are and no positions are kept: the order
+// of A's device lists.
 struct SpreadArgs {
     const int32_t* ptr[2];
     const uint32_t* ent0[2];
@@ -100,13 +103,15 @@ struct SpreadArgs {
     int32_t n;
 };
 
+template <bool RELABEL>
 __device__ __forceinline__ void spread_place(const uint32_t* __restrict__ ent0, const int32_t* __restrict__ pinv,
                                              uint32_t* __restrict__ ent, int32_t* __restrict__ pos, int32_t i, int32_t at) {
     const uint32_t e = __ldg(ent0 + i);
-    ent[at] = bm_pack((uint32_t)__ldg(pinv + bm_eid(e)), (uint32_t)bm_ew(e));
-    pos[i] = at;
+    ent[at] = RELABEL ? bm_pack((uint32_t)__ldg(pinv + bm_eid(e)), (uint32_t)bm_ew(e)) : e;
+    if (RELABEL) pos[i] = at;
 }
 
+template <bool RELABEL>
 __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
     const int lane = threadIdx.x & 31;
     const int dir = blockIdx.y;
@@ -116,6 +121,7 @@ __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
     int32_t* __restrict__ pos = a.pos[dir];
     int32_t* tmp = a.tmp[dir];
     const int32_t* __restrict__ pinv = a.pinv;
+    auto bank_of = [pinv](uint32_t e) { return (RELABEL ? __ldg(pinv + bm_eid(e)) : bm_eid(e)) & 31; };
     for (int32_t g = blockIdx.x * 8 + (threadIdx.x >> 5); g <= a.n; g += gridDim.x * 8) {
         const int32_t lo = __ldg(ent_ptr + g), hi = __ldg(ent_ptr + g + 1);
         if (lo == hi) continue;
@@ -125,7 +131,7 @@ __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
         int32_t num = 0;  // of bank `lane`
         for (int32_t i0 = lo; i0 < lo + cnt; i0 += 32) {
             const int32_t i = i0 + lane;
-            const int b = i < lo + cnt ? __ldg(pinv + bm_eid(__ldg(ent0 + i))) & 31 : 32;
+            const int b = i < lo + cnt ? bank_of(__ldg(ent0 + i)) : 32;
             const unsigned same = __match_any_sync(0xffffffffu, b);
             const int leader = __ffs(same) - 1;
             // the leader of every bank present tells its lane the count
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
         int32_t head = start;
         for (int32_t i0 = lo; i0 < lo + cnt; i0 += 32) {
             const int32_t i = i0 + lane;
-            const int b = i < lo + cnt ? __ldg(pinv + bm_eid(__ldg(ent0 + i))) & 31 : 32;
+            const int b = i < lo + cnt ? bank_of(__ldg(ent0 + i)) : 32;
             const unsigned same = __match_any_sync(0xffffffffu, b);
             const int32_t at = __shfl_sync(0xffffffffu, head, b & 31) + __popc(same & ((1u << lane) - 1u));
             if (b < 32) tmp[at] = i;
@@ -165,7 +171,7 @@ __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
 #pragma unroll
             for (int o = 0; o < 4; o++) r += ((b - 8 * o) & 31) < q;
             const int32_t s = __shfl_sync(0xffffffffu, start, b);
-            spread_place(ent0, pinv, ent, pos, tmp[s + 4 * (p >> 7) + r], lo + p);
+            spread_place<RELABEL>(ent0, pinv, ent, pos, tmp[s + 4 * (p >> 7) + r], lo + p);
         }
         // the rest in order
         int32_t left = num - 4 * turns, at = start + 4 * turns;
@@ -182,9 +188,12 @@ __global__ void __launch_bounds__(256) spread_relabel_kernel(SpreadArgs a) {
                 if (lane == b) { at++; left--; }
                 avail = __ballot_sync(0xffffffffu, left > 0);
             }
-            if (lane < steps) spread_place(ent0, pinv, ent, pos, tmp[mine], lo + p0 + lane);
+            if (lane < steps) spread_place<RELABEL>(ent0, pinv, ent, pos, tmp[mine], lo + p0 + lane);
         }
-        for (int32_t j = lo + cnt + lane; j < hi; j += 32) { ent[j] = 0u; pos[j] = j; }
+        for (int32_t j = lo + cnt + lane; j < hi; j += 32) {
+            ent[j] = 0u;
+            if (RELABEL) pos[j] = j;
+        }
         __syncwarp();
     }
 }
@@ -244,6 +253,19 @@ bm_status bm_check_score(bm_ctx* ctx) {
     return BM_OK;
 }
 
+bm_status bm_launch_spread(bm_ctx* ctx, int32_t n, const int32_t* optr, const int32_t* iptr, const uint32_t* oent,
+                           const uint32_t* ient, uint32_t* out, uint32_t* in, int32_t* tmp) {
+    const unsigned blocks = (unsigned)std::min((n + 8) / 8, ctx->num_sms * 8);
+    // one direction after the other: they share tmp
+    const SpreadArgs so{{optr, optr}, {oent, oent}, {out, out}, {nullptr, nullptr}, {tmp, tmp}, nullptr, n};
+    spread_relabel_kernel<false><<<blocks, 256, 0, ctx->stream>>>(so);
+    BM_LAUNCH_CHECK(ctx, "spread_kernel(out)");
+    const SpreadArgs si{{iptr, iptr}, {ient, ient}, {in, in}, {nullptr, nullptr}, {tmp, tmp}, nullptr, n};
+    spread_relabel_kernel<false><<<blocks, 256, 0, ctx->stream>>>(si);
+    BM_LAUNCH_CHECK(ctx, "spread_kernel(in)");
+    return BM_OK;
+}
+
 bm_status bm_launch_relabel(bm_ctx* ctx) {
     const DevGraph& B = ctx->g[1];
     image_bounds_kernel<<<(ctx->n + 1 + 255) / 256, 256, 0, ctx->stream>>>(ctx->pi, B.in_ptr, B.out_ptr, ctx->n, ctx->ximg);
@@ -252,7 +274,8 @@ bm_status bm_launch_relabel(bm_ctx* ctx) {
     // the live twin arrays serve as the placement scratch, then are rebuilt
     const SpreadArgs sa{{B.out_ptr, B.in_ptr},   {B.out_ent0, B.in_ent0}, {B.out_ent, B.in_ent},
                         {B.out_pos, B.in_pos},   {B.out_twin, B.in_twin}, ctx->pinv, ctx->n};
-    spread_relabel_kernel<<<dim3((unsigned)std::min((ctx->n + 8) / 8, ctx->num_sms * 8), 2), 256, 0, ctx->stream>>>(sa);
+    spread_relabel_kernel<true>
+        <<<dim3((unsigned)std::min((ctx->n + 8) / 8, ctx->num_sms * 8), 2), 256, 0, ctx->stream>>>(sa);
     BM_LAUNCH_CHECK(ctx, "spread_relabel_kernel");
     const int tb = ctx->num_sms * 4;
     if (B.m_out > 0) {
