@@ -85,88 +85,56 @@ constexpr int kSaMaxK = 64;         // proposals per iteration, adaptive up to t
 constexpr int kSaMaxInitialK = 16;  // largest settable starting K
 constexpr int kSaItem = 128;        // list entries per work item (four per lane)
 constexpr int kSaRowCap = 512;      // B row entries a warp stages in shared memory (longer rows: hash)
+constexpr int kSaSlots = 2048;      // slots of a warp's index of its staged row (a byte each)
+constexpr int kSaIndexed = 252;     // longest indexed row (slot values 1..252; 255: shared by two entries)
 constexpr int kSaUnitTable = 4096;  // items per iteration with an item -> list table (else binary search)
 
-constexpr int kSaApplyRowCap = 4096;  // entries per staged row in the swap apply (4 rows)
-
 // Dynamic shared memory of the chain kernel: the warps' B-row buffers (two
-// per warp), which the swap apply reuses for its four staged rows (at least
-// 64 KB), then the chain's mapping when it fits.
+// per warp) and row indexes, then the chain's mapping when it fits.
+__host__ __device__ constexpr size_t sa_rows_bytes(int threads) {
+    return sizeof(uint32_t) * kSaRowCap * 2 * (size_t)(threads / 32);
+}
 __host__ __device__ constexpr size_t sa_dyn_base(int threads) {
-    return sizeof(uint32_t) * kSaRowCap * 2 * (size_t)(threads / 32) > sizeof(uint32_t) * 4 * kSaApplyRowCap
-               ? sizeof(uint32_t) * kSaRowCap * 2 * (size_t)(threads / 32)
-               : sizeof(uint32_t) * 4 * kSaApplyRowCap;
+    return sa_rows_bytes(threads) + (size_t)kSaSlots * (size_t)(threads / 32);
 }
 
 // Apply the swap pi(a) <-> pi(b) of one chain with the whole CTA: S updates of
 // every A entry incident to a or b (as apply_kernel in bm_apply.cu), then pi.
-// Every lookup is in one of four B rows (out and in of pi a and pi b), staged
-// in `stage` (4 x kSaApplyRowCap entries of shared memory; longer rows use
-// the hash).  `pi` is the working copy (shared or global memory), `gpi` the
-// chain's mapping in global memory, updated too.
+// The four lists are one stream of entries over the chain's threads, each entry
+// two independent hash lookups: one trip for all but hubs, where staging B's
+// rows first and searching them list by list took 15,000 cycles a swap.
+// `pi` is the working copy (shared or global memory), `gpi` the chain's mapping
+// in global memory, updated too.
 template <int CL>
 __device__ void chain_apply_block(const PairDev& P, int32_t* pi, int32_t* gpi, int32_t* ov, int32_t sa, int32_t sb,
-                                  uint32_t* stage, int crank) {
+                                  int crank) {
     const int32_t fa = pi[sa], fb = pi[sb];
-    // rows: 0 = out(fa), 1 = out(fb), 2 = in(fa), 3 = in(fb)
-    int32_t rlen[4];
-    bool rst[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        const int32_t g = (r & 1) ? fb : fa;
-        const int32_t* ptr = (r < 2) ? P.Bout_ptr : P.Bin_ptr;
-        const uint32_t* ent = (r < 2) ? P.Bout_ent : P.Bin_ent;
-        const int32_t b = __ldg(ptr + g);
-        rlen[r] = __ldg(ptr + g + 1) - b;
-        rst[r] = rlen[r] <= kSaApplyRowCap;
-        if (rst[r])
-            for (int32_t j = threadIdx.x; j < rlen[r]; j += blockDim.x) stage[r * kSaApplyRowCap + j] = __ldg(ent + b + j);
-    }
-    __syncthreads();
-    // B(g, h) for g in {fa, fb} (rows 0, 1) and B(h, g) (rows 2, 3)
-    auto bout = [&](int32_t g, int32_t h) -> int32_t {
-        const bool a = g == fa;
-        const int32_t len = a ? rlen[0] : rlen[1];
-        const bool st = a ? rst[0] : rst[1];
-        return st ? bm_row_weight(stage + (a ? 0 : kSaApplyRowCap), len, h) : bm_hash_get(P.hb, g, h);
-    };
-    auto bin = [&](int32_t h, int32_t g) -> int32_t {
-        const bool a = g == fa;
-        const int32_t len = a ? rlen[2] : rlen[3];
-        const bool st = a ? rst[2] : rst[3];
-        return st ? bm_row_weight(stage + (a ? 2 : 3) * kSaApplyRowCap, len, h) : bm_hash_get(P.hb, h, g);
-    };
-    for (int side = 0; side < 2; side++) {
-        const int32_t me = side ? sb : sa, other = side ? sa : sb;
-        const int32_t fme = side ? fb : fa, fnew = side ? fa : fb;
-        {
-            const int32_t b = __ldg(P.Aout_ptr + me), e = __ldg(P.Aout_ptr + me + 1);
-            for (int32_t j = b + (int32_t)threadIdx.x + crank * (int32_t)blockDim.x; j < e; j += CL * (int32_t)blockDim.x) {
-                const uint32_t ent = __ldg(P.Aout_ent + j);
-                if (ent == 0) continue;
-                const int32_t x = bm_eid(ent), w = bm_ew(ent);
-                if (x == other) {
-                    const int32_t d = imin(w, bout(fnew, fme)) - imin(w, bout(fme, fnew));
-                    if (d) { atomicAdd(ov + me, d); atomicAdd(ov + other, d); }
-                } else {
-                    const int32_t gx = pi[x];
-                    const int32_t d = imin(w, bout(fnew, gx)) - imin(w, bout(fme, gx));
-                    if (d) { atomicAdd(ov + me, d); atomicAdd(ov + x, d); }
-                }
-            }
+    const int32_t o0 = __ldg(P.Aout_ptr + sa), o1 = __ldg(P.Aout_ptr + sa + 1);
+    const int32_t i0 = __ldg(P.Ain_ptr + sa), i1 = __ldg(P.Ain_ptr + sa + 1);
+    const int32_t p0 = __ldg(P.Aout_ptr + sb), p1 = __ldg(P.Aout_ptr + sb + 1);
+    const int32_t q0 = __ldg(P.Ain_ptr + sb), q1 = __ldg(P.Ain_ptr + sb + 1);
+    // running ends of out(sa), in(sa), out(sb), in(sb)
+    const int32_t e0 = o1 - o0, e1 = e0 + (i1 - i0), e2 = e1 + (p1 - p0), e3 = e2 + (q1 - q0);
+#pragma unroll 2
+    for (int32_t j = (int32_t)threadIdx.x + crank * (int32_t)blockDim.x; j < e3; j += CL * (int32_t)blockDim.x) {
+        const bool of_a = j < e1, out = j < e0 || (j >= e1 && j < e2);
+        const int32_t at = j + (of_a ? (out ? o0 : i0 - e0) : (out ? p0 - e1 : q0 - e2));
+        const uint32_t ent = __ldg((out ? P.Aout_ent : P.Ain_ent) + at);
+        if (ent == 0) continue;
+        const int32_t x = bm_eid(ent), w = bm_ew(ent);
+        const int32_t me = of_a ? sa : sb, other = of_a ? sb : sa;
+        const int32_t fme = of_a ? fa : fb, fnew = of_a ? fb : fa;
+        int32_t g0, h0, g1, h1;  // B edge before and after
+        if (x == other) {
+            if (!out) continue;  // the edge other -> me is handled as other's out-entry
+            g0 = fme; h0 = fnew; g1 = fnew; h1 = fme;
+        } else {
+            const int32_t gx = pi[x];
+            g0 = out ? fme : gx; h0 = out ? gx : fme;
+            g1 = out ? fnew : gx; h1 = out ? gx : fnew;
         }
-        {
-            const int32_t b = __ldg(P.Ain_ptr + me), e = __ldg(P.Ain_ptr + me + 1);
-            for (int32_t j = b + (int32_t)threadIdx.x + crank * (int32_t)blockDim.x; j < e; j += CL * (int32_t)blockDim.x) {
-                const uint32_t ent = __ldg(P.Ain_ent + j);
-                if (ent == 0) continue;
-                const int32_t x = bm_eid(ent), w = bm_ew(ent);
-                if (x == other) continue;
-                const int32_t gx = pi[x];
-                const int32_t d = imin(w, bin(gx, fnew)) - imin(w, bin(gx, fme));
-                if (d) { atomicAdd(ov + me, d); atomicAdd(ov + x, d); }
-            }
-        }
+        const int32_t d = imin(w, bm_hash_get(P.hb, g1, h1)) - imin(w, bm_hash_get(P.hb, g0, h0));
+        if (d) { atomicAdd(ov + me, d); atomicAdd(ov + x, d); }
     }
     // every read of the mapping (both CTAs of a pair) before it changes
     if constexpr (CL > 1) cg::this_cluster().sync(); else __syncthreads();
@@ -193,8 +161,14 @@ __device__ void chain_apply_block(const PairDev& P, int32_t* pi, int32_t* gpi, i
 // so every entry of one list looks up the same B row (B-out or B-in of pi v
 // or pi u).  The lists are cut into items of kSaItem entries; warp w takes
 // items w, w + 16, ..., stages the item's B row in its shared buffer with
-// coalesced loads, and each lane binary-searches pi x in it (rows longer
-// than the buffer use the hash).  For an entry of u whose other end is v,
+// coalesced loads, enters the row's positions in a small index by the low bits
+// of the id, and each lane reads pi x there: three dependent shared-memory
+// reads, where a binary search of the row took seven to nine, and most end at
+// an empty slot.  (Rows of more than 252 entries are searched, rows longer
+// than the buffer use the hash; a slot that two entries of the row share is
+// marked and searched.)  64 chains of 100,000 steps on four pairs of 2,709 to
+// 8,192 vertices: 107 ms with the searches and the staged swap apply, 89 ms so;
+// what bounds an iteration now is the latency of its 16 warps an SM.  For an entry of u whose other end is v,
 // the direct-edge repair min(w, B(pi u, pi v)) + min(w, B(pi v, pi u)) is
 // added; the item sums meet in a per-proposal shared counter, then
 //   delta = sum - S(u) - S(v) + self-loop terms.
@@ -217,6 +191,8 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
     __shared__ bm_proposal s_prop[kSaMaxK];
     __shared__ int32_t s_sum[kSaMaxK];
     __shared__ long long s_d[kSaMaxK];
+    __shared__ int32_t s_ov[2][kSaMaxK];           // S(u), S(v) of the proposals
+    __shared__ double s_temp[kSaMaxK];
     __shared__ int32_t s_seglen[kSeg];             // entries per list
     __shared__ int32_t s_segbase[kSeg];            // offset of each list in its CSR
     __shared__ int32_t s_upre[kSeg + 1];           // unit prefix over the lists
@@ -229,6 +205,10 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
     int32_t* gpi = ch.pi;
     int32_t* pi = gpi;
     uint32_t* rowbuf = s_dyn + (size_t)warp * 2 * kSaRowCap;  // this warp's two B-row buffers
+    // this warp's index of the row being searched: position + 1 by the id's low
+    // bits; all zero between items
+    uint8_t* slots = reinterpret_cast<uint8_t*>(s_dyn) + sa_rows_bytes(THREADS) + (size_t)warp * kSaSlots;
+    for (int32_t i = lane; i < kSaSlots / 16; i += 32) reinterpret_cast<uint4*>(slots)[i] = make_uint4(0u, 0u, 0u, 0u);
     if (a.pi_smem) {
         int32_t* s_pi = reinterpret_cast<int32_t*>(s_dyn + sa_dyn_base(THREADS) / sizeof(uint32_t));
         for (int32_t i = tid; i <= P.n; i += blockDim.x) s_pi[i] = gpi[i];
@@ -256,6 +236,9 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                 const int32_t* ptr = (kind & 1) ? P.Ain_ptr : P.Aout_ptr;
                 base = __ldg(ptr + me);
                 len = __ldg(ptr + me + 1) - base;
+                // what the decision needs besides the sums, off its path
+                if (kind & 1) s_ov[kind >> 1][w] = ov[me];
+                if (kind == 2) s_temp[w] = bm_sa_temperature(a.t0, a.log_ratio, sidx, a.steps);
             }
             s_seglen[tid] = len;
             s_segbase[tid] = base;
@@ -290,13 +273,13 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
         // warp's other buffer, and item i is searched, all at once
         {
             struct Stage {
-                int32_t item, w, kind, g, rb, rl;
+                int32_t item, w, kind, g, rb, re;  // B row [rb, re): no arithmetic on them until they are used
                 uint32_t ent[kSaItem / 32];
             };
             auto fetch = [&](int32_t item, Stage& st) {
                 st.item = item;
                 st.rb = 0;
-                st.rl = 0;
+                st.re = 0;
                 st.w = 0;
                 st.kind = 0;
                 st.g = 0;
@@ -328,14 +311,15 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                 st.g = st.kind < 2 ? pi[pr.v] : pi[pr.u];
                 const int32_t* rptr = out ? P.Bout_ptr : P.Bin_ptr;
                 st.rb = __ldg(rptr + st.g);
-                st.rl = __ldg(rptr + st.g + 1) - st.rb;
+                st.re = __ldg(rptr + st.g + 1);
             };
             // B rows start on 16-byte boundaries (rows are padded to multiples of 4)
             auto copy_row = [&](const Stage& st, int buf) {
-                if (st.item < U && st.rl <= kSaRowCap) {
+                const int32_t rl = st.re - st.rb;
+                if (st.item < U && rl <= kSaRowCap) {
                     const uint32_t* rent = !(st.kind & 1) ? P.Bout_ent : P.Bin_ent;
                     const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(rowbuf + (size_t)buf * kSaRowCap);
-                    for (int32_t j = 4 * lane; j < st.rl; j += 128)
+                    for (int32_t j = 4 * lane; j < rl; j += 128)
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst0 + 4u * (uint32_t)j),
                                      "l"(rent + st.rb + j) : "memory");
                 }
@@ -343,55 +327,124 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
             };
             constexpr int kStride = CL * kW;  // the chain's warps over all its CTAs
             const int gw = crank * kW + warp;
-            Stage cur, nxt, far;
-            fetch(gw, cur);
-            fetch(gw + kStride, nxt);
-            copy_row(cur, 0);
-            int buf = 0;
-            for (int32_t item = gw; item < U; item += kStride) {
+            // the stages take turns in three roles instead of being copied: a
+            // copy of a register that a load is still filling waits for the load
+            auto search = [&](int32_t item, const Stage& cur, const Stage& nxt, Stage& far, int buf) {
                 copy_row(nxt, buf ^ 1);
                 fetch(item + 2 * kStride, far);
                 asm volatile("cp.async.wait_group 1;" ::: "memory");  // this item's row has landed
                 __syncwarp();
                 const uint32_t* row = rowbuf + (size_t)buf * kSaRowCap;
                 const bool out = !(cur.kind & 1);
-                const bool staged = cur.rl <= kSaRowCap;
+                const int32_t rl = cur.re - cur.rb;
+                const bool staged = rl <= kSaRowCap;
                 const bm_proposal pr = s_prop[cur.w];
+                const bool indexed = rl <= kSaIndexed;
+                // rows are whole quads: position j of the row goes to slot id mod
+                // kSaSlots; where two meet, the one that lost marks the slot
+                if (indexed) {
+                    for (int32_t q = lane; q < rl / 4; q += 32) {
+                        const uint4 e = reinterpret_cast<const uint4*>(row)[q];
+                        const uint32_t v[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            if (v[k]) slots[bm_eid(v[k]) & (kSaSlots - 1)] = (uint8_t)(4 * q + k + 1);
+                    }
+                    __syncwarp();
+                    for (int32_t q = lane; q < rl / 4; q += 32) {
+                        const uint4 e = reinterpret_cast<const uint4*>(row)[q];
+                        const uint32_t v[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            uint8_t* s = slots + (bm_eid(v[k]) & (kSaSlots - 1));
+                            if (v[k] && *s != (uint8_t)(4 * q + k + 1)) *s = 255;
+                        }
+                    }
+                    __syncwarp();
+                }
                 int32_t val = 0;
+                int32_t gx4[kSaItem / 32], at4[kSaItem / 32], wb4[kSaItem / 32];
+#pragma unroll
+                for (int k = 0; k < kSaItem / 32; k++) gx4[k] = pi[bm_eid(cur.ent[k])];
+#pragma unroll
+                for (int k = 0; k < kSaItem / 32; k++) at4[k] = indexed ? slots[gx4[k] & (kSaSlots - 1)] : 255;
+                if (staged) {
+#pragma unroll
+                    for (int k = 0; k < kSaItem / 32; k++) {
+                        if (at4[k] != 255) {
+                            const uint32_t e = at4[k] ? row[at4[k] - 1] : 0u;
+                            wb4[k] = bm_eid(e) == gx4[k] ? bm_ew(e) : 0;
+                        } else {
+                            wb4[k] = cur.ent[k] ? bm_row_weight(row, rl, gx4[k]) : 0;
+                        }
+                    }
+                } else {
+                    // the lane's lookups in flight together: the first group of
+                    // slots of each, then the few that it does not settle
+                    ulonglong2 s0[kSaItem / 32], s1[kSaItem / 32];
+                    const unsigned long long np1 = (unsigned long long)P.hb.np1;
+#pragma unroll
+                    for (int k = 0; k < kSaItem / 32; k++) {
+                        const int32_t g = out ? cur.g : gx4[k], h = out ? gx4[k] : cur.g;
+                        const unsigned long long key = (unsigned long long)g * np1 + (unsigned long long)h;
+                        const ulonglong2* p =
+                            reinterpret_cast<const ulonglong2*>(P.hb.tab + (bm_hash_slot0(key, P.hb.log2) & ~3ull));
+                        s0[k] = cur.ent[k] ? __ldg(p) : make_ulonglong2(0, 0);
+                        s1[k] = cur.ent[k] ? __ldg(p + 1) : make_ulonglong2(0, 0);
+                    }
+#pragma unroll
+                    for (int k = 0; k < kSaItem / 32; k++) {
+                        wb4[k] = 0;
+                        if (cur.ent[k] == 0) continue;
+                        const int32_t g = out ? cur.g : gx4[k], h = out ? gx4[k] : cur.g;
+                        const unsigned long long key = (unsigned long long)g * np1 + (unsigned long long)h;
+                        const int from = (int)(bm_hash_slot0(key, P.hb.log2) & 3ull);
+                        const unsigned long long v[4] = {s0[k].x, s0[k].y, s1[k].x, s1[k].y};
+                        bool settled = false;
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (q < from || settled) continue;
+                            if (v[q] == BM_HASH_EMPTY) settled = true;
+                            else if ((v[q] >> 16) == key) { wb4[k] = (int32_t)(v[q] & 0xFFFFull); settled = true; }
+                        }
+                        if (!settled) wb4[k] = bm_hash_get(P.hb, g, h);
+                    }
+                }
 #pragma unroll
                 for (int k = 0; k < kSaItem / 32; k++) {
                     if (cur.ent[k] == 0) continue;
                     const int32_t x = bm_eid(cur.ent[k]), wa = bm_ew(cur.ent[k]);
-                    const int32_t gx = pi[x];
-                    int32_t wb = 0;
-                    if (staged) {
-                        // first row slot whose id is >= gx (zero padding sorts last)
-                        int32_t l = 0, h = cur.rl;
-                        while (l < h) {
-                            const int32_t mid = (l + h) >> 1;
-                            const uint32_t e = row[mid];
-                            if (e != 0u && bm_eid(e) < gx) l = mid + 1; else h = mid;
-                        }
-                        if (l < cur.rl) {
-                            const uint32_t e = row[l];
-                            if (e != 0u && bm_eid(e) == gx) wb = bm_ew(e);
-                        }
-                    } else {
-                        wb = out ? bm_hash_get(P.hb, cur.g, gx) : bm_hash_get(P.hb, gx, cur.g);
-                    }
-                    val += imin(wa, wb);
+                    val += imin(wa, wb4[k]);
                     if (cur.kind < 2 && x == pr.v) {
                         const int32_t fu = pi[pr.u], fv = pi[pr.v];
                         val += imin(wa, bm_hash_get(P.hb, fu, fv)) + imin(wa, bm_hash_get(P.hb, fv, fu));
                     }
                 }
-                // an item lies in one list, hence one proposal: warp sum, one atomic
+                if (indexed) {
+                    __syncwarp();  // every lane has read the index
+                    for (int32_t q = lane; q < rl / 4; q += 32) {
+                        const uint4 e = reinterpret_cast<const uint4*>(row)[q];
+                        const uint32_t v[4] = {e.x, e.y, e.z, e.w};
 #pragma unroll
-                for (int o = 16; o; o >>= 1) val += __shfl_xor_sync(0xffffffffu, val, o);
+                        for (int k = 0; k < 4; k++) slots[bm_eid(v[k]) & (kSaSlots - 1)] = 0;
+                    }
+                }
+                // an item lies in one list, hence one proposal: warp sum, one atomic
+                val = __reduce_add_sync(0xffffffffu, val);
                 if (lane == 0 && val) atomicAdd(&s_sum[cur.w], val);
                 __syncwarp();  // this buffer is rewritten two items on
-                cur = nxt;
-                nxt = far;
+            };
+            Stage s0, s1, s2;
+            fetch(gw, s0);
+            fetch(gw + kStride, s1);
+            copy_row(s0, 0);
+            int buf = 0;
+            for (int32_t item = gw; item < U; item += 3 * kStride) {
+                search(item, s0, s1, s2, buf);
+                if (item + kStride >= U) break;
+                search(item + kStride, s1, s2, s0, buf ^ 1);
+                if (item + 2 * kStride >= U) break;
+                search(item + 2 * kStride, s2, s0, s1, buf);
                 buf ^= 1;
             }
             asm volatile("cp.async.wait_all;" ::: "memory");
@@ -408,7 +461,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
 #pragma unroll
                 for (int q = 1; q < CL; q++) sum += *cg::this_cluster().map_shared_rank(s_sum + tid, (crank + q) % CL);
             }
-            long long d = sum - (long long)ov[pr.u] - (long long)ov[pr.v];
+            long long d = sum - (long long)s_ov[0][tid] - (long long)s_ov[1][tid];
             if (P.has_self) {
                 const int32_t fu = pi[pr.u], fv = pi[pr.v];
                 const int32_t su = __ldg(P.selfA + pr.u), sv = __ldg(P.selfA + pr.v);
@@ -416,7 +469,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                 d += imin(su, bv) - imin(su, bu) + imin(sv, bu) - imin(sv, bv);
             }
             s_d[tid] = d;
-            if (bm_sa_accept(d, pr.uni, bm_sa_temperature(a.t0, a.log_ratio, step + (uint64_t)tid, a.steps)))
+            if (bm_sa_accept(d, pr.uni, s_temp[tid]))
                 atomicMin(&s_first, tid);
         }
         __syncthreads();
@@ -427,7 +480,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
             accepts++;
             step += (uint64_t)first + 1;
             K = min(kSaMaxK, max(a.K, 2 * (first + 1)));
-            chain_apply_block<CL>(P, pi, gpi, ov, pr.u, pr.v, s_dyn, crank);  // ends with a (cluster) barrier
+            chain_apply_block<CL>(P, pi, gpi, ov, pr.u, pr.v, crank);  // ends with a (cluster) barrier
             if (tid == 0) s_first = kSaMaxK;
         } else {
             step = min(end, step + (uint64_t)K);
