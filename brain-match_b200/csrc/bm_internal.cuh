@@ -365,7 +365,11 @@ bm_status bm_launch_rows_ex(bm_ctx* ctx, const int32_t* d_rows, const int32_t* d
 // of u alone taking v's image with every other vertex fixed.
 bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* d_col_lo, int32_t nrows,
                              int64_t* d_full, bm_row_result* d_res, int32_t* d_tab, int64_t tab_ld, int32_t tab_sym,
-                             const int32_t* d_cols, int32_t ncols, int32_t* d_colout, const int32_t* h_rows = nullptr);
+                             const int32_t* d_cols, int32_t ncols, int32_t* d_colout, const int32_t* h_rows = nullptr,
+                             bool gains = false);
+// gains: the one-sided sums of whole rows, d_tab[u * tab_ld + v] = G_u(pi v)
+// (d_tab 16-byte aligned, tab_ld a multiple of 4 and at least n + 1): half the
+// scatter of a delta row, whose other half is G_v(pi u).
 bm_status bm_launch_apply(bm_ctx* ctx, const int32_t* d_pairs, int32_t k);
 bm_status bm_rows_smem_check(bm_ctx* ctx);
 bm_status bm_launch_kset(bm_ctx* ctx, int32_t k, const int32_t* d_sets, int64_t nsets, long long* d_best,

@@ -98,7 +98,8 @@ struct RowArgs {
     int32_t tab_sym;   // also write entry (v, u)
     // one-sided mode: only T1 + T2 (u's own edges moved to pi v, everything
     // else fixed), read at the columns cols[0..ncols): colout[r * ncols + j] =
-    // G_u(pi cols[j]) - S(u) + self-loop term
+    // G_u(pi cols[j]) - S(u) + self-loop term; without cols, the bare sums of
+    // every column go to the table: tab[u * tab_ld + v] = G_u(pi v)
     int32_t half;
     const int32_t* cols;
     int32_t ncols;
@@ -164,9 +165,10 @@ __device__ __forceinline__ bm_row_result row_result(int32_t u, const Partial& t)
     return out;
 }
 
-// REFCPU: reference-delta semantics (a separate instantiation, so the exact
-// one carries none of its code or registers)
-template <int THREADS, bool REFCPU>
+// REFCPU: reference-delta semantics; GAINS: one-sided sums of whole rows into
+// the table (separate instantiations, so the exact one carries none of their
+// code or registers)
+template <int THREADS, bool REFCPU, bool GAINS>
 __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
     constexpr int NW = THREADS / 32;
     constexpr int IPT = kItemChunk / THREADS;  // items built per thread
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
         const int32_t ai = __ldg(a.Ain_ptr + u), d2 = __ldg(a.Ain_ptr + u + 1) - ai;
         const int32_t bo = __ldg(a.Bout_ptr + fu), d3 = __ldg(a.Bout_ptr + fu + 1) - bo;
         const int32_t bi = __ldg(a.Bin_ptr + fu), d4 = __ldg(a.Bin_ptr + fu + 1) - bi;
-        const int32_t F = a.half ? d1 + d2 : d1 + d2 + d3 + d4;
+        const int32_t F = GAINS || a.half ? d1 + d2 : d1 + d2 + d3 + d4;
         const int32_t dA = d1 + d2;
         // ---- direct-edge corrections C, for A entries (x, w) of u:
         //   acc[x] += min(w, B(pi u, pi x)) + min(w, B(pi x, pi u)).
@@ -285,7 +287,7 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
         // more than kSideCap A entries use hash lookups, spread over the
         // cluster's CTAs.
         const bool side_path = dA <= kSideCap;
-        if (!a.half && side_path && crank == 0 && P(1) == 0) {
+        if (!GAINS && !a.half && side_path && crank == 0 && P(1) == 0) {
             int32_t* side = reinterpret_cast<int32_t*>(it_base);
             for (int32_t j = tid; j < d3; j += THREADS) {
                 const uint32_t e = __ldg(a.Bout_ent + bo + j);
@@ -361,7 +363,7 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
                             len = xb.w - xb.z;
                         }
                         cap = w;
-                        if (!a.half && !side_path && (i % CL) == crank) {
+                        if (!GAINS && !a.half && !side_path && (i % CL) == crank) {
                             const int32_t g = __ldg(a.pi + x);
                             const int32_t c = imin(w, bm_hash_get_small(a.hb, fu, g)) + imin(w, bm_hash_get_small(a.hb, g, fu));
                             if (c) atomicAdd(acc + x, c);
@@ -573,6 +575,23 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
             a.colout[(size_t)r * (size_t)a.ncols + j] = (int32_t)c;
         }
     }
+    if constexpr (GAINS) {
+        // gain table: 16-byte aligned rows (checked by the launcher); columns
+        // past n are not the table's
+        int32_t* trow = a.tab + (size_t)u * (size_t)a.tab_ld;
+        for (int32_t gi = glo + tid; valid && gi < ghi; gi += THREADS) {
+            const int4 s4 = cluster_sum(gi);
+            if (4 * gi + 3 <= n) {
+                reinterpret_cast<int4*>(trow)[gi] = s4;
+            } else {
+                trow[4 * gi] = s4.x;
+                if (4 * gi + 1 <= n) trow[4 * gi + 1] = s4.y;
+                if (4 * gi + 2 <= n) trow[4 * gi + 2] = s4.z;
+            }
+        }
+        cluster.sync();  // the other CTAs' sums are read no more
+        return;
+    }
     auto finish_group = [&](int32_t gi, const int4 s4) {
         const int4 o4 = __ldg(ov4 + gi);
         const int32_t sv[4] = {s4.x, s4.y, s4.z, s4.w};
@@ -742,10 +761,10 @@ __global__ void __launch_bounds__(kWorkThreads) row_work_kernel(RowArgs a, int32
     if (lane == 0) work[u] = (int32_t)min(s, (long long)INT_MAX);
 }
 
-template <int THREADS, bool REFCPU>
+template <int THREADS, bool REFCPU, bool GAINS = false>
 bm_status launch_rows_t(bm_ctx* ctx, const RowArgs& args, int cl, size_t smem, cudaStream_t stream) {
     static bool configured[64] = {false};
-    auto kern = rows_kernel<THREADS, REFCPU>;
+    auto kern = rows_kernel<THREADS, REFCPU, GAINS>;
     if (!configured[ctx->device & 63]) {
         BM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
         configured[ctx->device & 63] = true;
@@ -774,7 +793,7 @@ bm_status launch_rows_t(bm_ctx* ctx, const RowArgs& args, int cl, size_t smem, c
 
 template <int THREADS>
 bm_status max_clusters_t(bm_ctx* ctx, int cl, size_t smem, int* out) {
-    auto kern = rows_kernel<THREADS, false>;
+    auto kern = rows_kernel<THREADS, false, false>;
     BM_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ctx->smem_optin));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(cl * 64), 1, 1);
@@ -947,7 +966,7 @@ bm_status bm_launch_rows_ex(bm_ctx* ctx, const int32_t* d_rows, const int32_t* d
 
 bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* d_col_lo, int32_t nrows,
                              int64_t* d_full, bm_row_result* d_res, int32_t* d_tab, int64_t tab_ld, int32_t tab_sym,
-                             const int32_t* d_cols, int32_t ncols, int32_t* d_colout, const int32_t* h_rows) {
+                             const int32_t* d_cols, int32_t ncols, int32_t* d_colout, const int32_t* h_rows, bool gains) {
     if (nrows <= 0) return BM_OK;
     bm_status st = bm_rows_smem_check(ctx);
     if (st != BM_OK) return st;
@@ -966,7 +985,7 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
     args.selfA = A.self_w;
     args.selfB = B.self_w;
     // one-sided gains (d_cols) are not swaps: they keep the exact rule
-    args.refcpu = (ctx->semantics == BM_SEMANTICS_REF_CPU && !d_cols) ? 1 : 0;
+    args.refcpu = (ctx->semantics == BM_SEMANTICS_REF_CPU && !d_cols && !gains) ? 1 : 0;
     args.has_self = args.refcpu ? A.has_self : (A.has_self && B.has_self);
     args.hb = hview(B);
     args.pi = ctx->pi;
@@ -980,7 +999,7 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
     args.tab = d_tab;
     args.tab_ld = tab_ld;
     args.tab_sym = tab_sym;
-    args.half = d_cols ? 1 : 0;
+    args.half = d_cols || gains ? 1 : 0;
     args.cols = d_cols;
     args.ncols = ncols;
     args.colout = d_colout;
@@ -996,7 +1015,7 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
     args.scnt = ctx->scnt;
     args.rcnt = ctx->rcnt;
     args.rpart = (Partial*)ctx->rpart;
-    if (h_rows && ctx->row_split >= 0 && !d_cols && ctx->slots && nrows < ctx->split_slots_max &&
+    if (h_rows && ctx->row_split >= 0 && !args.half && ctx->slots && nrows < ctx->split_slots_max &&
         ctx->h_rwork.size() == (size_t)ctx->n + 1) {
         // slots: the resident clusters of this shape when they are at least
         // four times the rows (automatic: launches of a few rows, where most
@@ -1032,6 +1051,9 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
         }
     }
     auto launch = [&](const RowArgs& x, int c, cudaStream_t strm) -> bm_status {
+        if (gains)
+            return (ctx->row_threads == 256) ? launch_rows_t<256, false, true>(ctx, x, c, smem, strm)
+                                             : launch_rows_t<512, false, true>(ctx, x, c, smem, strm);
         if (x.refcpu)
             return (ctx->row_threads == 256) ? launch_rows_t<256, true>(ctx, x, c, smem, strm)
                                              : launch_rows_t<512, true>(ctx, x, c, smem, strm);

@@ -334,6 +334,119 @@ __global__ void __launch_bounds__(1024) rank_sort_kernel(Sel sel, const TopState
     }
 }
 
+// ---------------------------------------------- deltas from one-sided gains
+//
+// delta(u, v) = G_u(pi v) + G_v(pi u) - S(u) - S(v) + self-loop terms + the
+// repair of direct edges.  The row kernel scatters both gains for every row;
+// over a whole table each gain is another row's other half, so the table is
+// filled with G_u(pi v) alone (half the scatter, which is what bounds the
+// table), and tile_sum_kernel adds it to its transpose in place, a pair of
+// 64 x 64 tiles a block, one read and one write of the table.  Then
+// repair_kernel adds the direct edges.  n = 18,524: 6.9 ms with both halves
+// scattered, 4.0 ms so (3.3 the scatter, 0.63 the sums, 0.11 the repair).
+constexpr int kTile = 64;
+
+struct SumArgs {
+    int32_t* tab;
+    int64_t ld;
+    int32_t n;
+    const int32_t* ov;
+    int has_self;
+    const int32_t* selfA;
+    const int32_t* selfB;
+    const int32_t* pi;
+};
+
+__global__ void __launch_bounds__(256) tile_sum_kernel(SumArgs a) {
+    __shared__ int32_t X[kTile][kTile + 1], Y[kTile][kTile + 1];
+    __shared__ int32_t s_ov[2][kTile], s_sa[2][kTile], s_sb[2][kTile];
+    // blocks enumerate the tile pairs I <= J of a triangle by rows
+    const int32_t T = (a.n + kTile) / kTile;  // tiles of rows 0..n
+    int32_t I, J;
+    {
+        const long long b = blockIdx.x;
+        I = (int32_t)(((2.0 * T + 1) - sqrt((2.0 * T + 1) * (2.0 * T + 1) - 8.0 * (double)b)) * 0.5);
+        auto first = [T](long long i) { return i * T - i * (i - 1) / 2; };
+        while (I > 0 && first(I) > b) I--;
+        while (first(I + 1) <= b) I++;
+        J = I + (int32_t)(b - first(I));
+    }
+    const int tid = threadIdx.x, c4 = tid & 15, r0 = tid >> 4;  // 16 threads of 4 columns, 16 rows a step
+    if (tid < 2 * kTile) {
+        const int side = tid / kTile, k = tid % kTile;
+        const int32_t v = (side ? J : I) * kTile + k;
+        s_ov[side][k] = v <= a.n ? __ldg(a.ov + v) : 0;
+        s_sa[side][k] = a.has_self && v >= 1 && v <= a.n ? __ldg(a.selfA + v) : 0;
+        s_sb[side][k] = a.has_self && v >= 1 && v <= a.n ? __ldg(a.selfB + __ldg(a.pi + v)) : 0;
+    }
+    const int4 zero = make_int4(0, 0, 0, 0);
+    for (int r = r0; r < kTile; r += 16) {
+        const int32_t u = I * kTile + r, w = J * kTile + r;
+        const int32_t cu = J * kTile + 4 * c4, cw = I * kTile + 4 * c4;  // ld covers whole groups up to n
+        const int4 x = u <= a.n && cu <= a.n ? *reinterpret_cast<const int4*>(a.tab + (size_t)u * a.ld + cu) : zero;
+        const int4 y = w <= a.n && cw <= a.n ? *reinterpret_cast<const int4*>(a.tab + (size_t)w * a.ld + cw) : zero;
+        X[r][4 * c4] = x.x; X[r][4 * c4 + 1] = x.y; X[r][4 * c4 + 2] = x.z; X[r][4 * c4 + 3] = x.w;
+        Y[r][4 * c4] = y.x; Y[r][4 * c4 + 1] = y.y; Y[r][4 * c4 + 2] = y.z; Y[r][4 * c4 + 3] = y.w;
+    }
+    __syncthreads();
+    // delta of row k of tile side s and column c of the other: symmetric
+    auto delta = [&](int i, int j) -> int32_t {  // u = I + i, v = J + j
+        const int32_t u = I * kTile + i, v = J * kTile + j;
+        if (u == v || u == 0 || v == 0) return 0;
+        int32_t d = X[i][j] + Y[j][i] - s_ov[0][i] - s_ov[1][j];
+        if (a.has_self)
+            d += imin(s_sa[0][i], s_sb[1][j]) - imin(s_sa[0][i], s_sb[0][i]) + imin(s_sa[1][j], s_sb[0][i]) -
+                 imin(s_sa[1][j], s_sb[1][j]);
+        return d;
+    };
+    auto store = [&](int32_t row, int32_t col, const int4 v) {
+        if (row > a.n || col > a.n) return;
+        int32_t* p = a.tab + (size_t)row * a.ld + col;
+        if (col + 3 <= a.n) {
+            *reinterpret_cast<int4*>(p) = v;
+        } else {
+            p[0] = v.x;
+            if (col + 1 <= a.n) p[1] = v.y;
+            if (col + 2 <= a.n) p[2] = v.z;
+        }
+    };
+    for (int r = r0; r < kTile; r += 16) {
+        const int c = 4 * c4;
+        store(I * kTile + r, J * kTile + c, make_int4(delta(r, c), delta(r, c + 1), delta(r, c + 2), delta(r, c + 3)));
+        if (I != J)
+            store(J * kTile + r, I * kTile + c, make_int4(delta(c, r), delta(c + 1, r), delta(c + 2, r), delta(c + 3, r)));
+    }
+}
+
+// The direct edges: an A entry u -> x of weight w adds min(w, B(pi u, pi x)) +
+// min(w, B(pi x, pi u)) to delta(u, x) and delta(x, u).  Warps take stretches
+// of 256 out-entries, whatever lists they fall in.
+__global__ void __launch_bounds__(256) repair_kernel(GView A, HashView hb, const int32_t* __restrict__ pi, int32_t n,
+                                                     int32_t* tab, int64_t ld) {
+    const int lane = threadIdx.x & 31;
+    const int32_t m = __ldg(A.out_ptr + n + 1);
+    for (int64_t c = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); c * 256 < m; c += (int64_t)gridDim.x * 8) {
+        const int32_t j0 = (int32_t)(c * 256), j1 = min(m, j0 + 256);
+        int32_t lo = 0, hi = n;  // the list that entry j0 falls in
+        while (lo < hi) {
+            const int32_t mid = (lo + hi + 1) >> 1;
+            if (__ldg(A.out_ptr + mid) <= j0) lo = mid; else hi = mid - 1;
+        }
+        int32_t u = lo, end = __ldg(A.out_ptr + u + 1);
+        for (int32_t j = j0 + lane; j < j1; j += 32) {
+            while (j >= end) end = __ldg(A.out_ptr + ++u + 1);
+            const uint32_t e = __ldg(A.out_ent + j);
+            if (!e) continue;  // list padding
+            const int32_t x = bm_eid(e), w = bm_ew(e), fu = __ldg(pi + u), fx = __ldg(pi + x);
+            const int32_t d = imin(w, bm_hash_get(hb, fu, fx)) + imin(w, bm_hash_get(hb, fx, fu));
+            if (d) {
+                atomicAdd(tab + (size_t)u * ld + x, d);
+                atomicAdd(tab + (size_t)x * ld + u, d);
+            }
+        }
+    }
+}
+
 __global__ void iota_kernel(int32_t* rows, int32_t n) {
     for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) rows[i] = i + 1;
 }
@@ -429,7 +542,26 @@ extern "C" bm_status bm_delta_table_dev(bm_ctx* ctx, int32_t* d_table, int64_t l
     BM_LAUNCH_CHECK(ctx, "iota_kernel");
     // row 0 is never written by the row kernel; keep it zero
     BM_CUDA(ctx, cudaMemsetAsync(d_table, 0, sizeof(int32_t) * (size_t)ld, ctx->stream));
-    return bm_launch_rows_ex(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0);
+    const DevGraph &A = ctx->g[0], &B = ctx->g[1];
+    // the reference-delta terms of self-loops are per row, and rows that do not
+    // start on 16-byte boundaries have no vector access: those keep the row
+    // kernel's own finish
+    const bool refcpu = ctx->semantics == BM_SEMANTICS_REF_CPU && A.has_self;
+    if (refcpu || (ld & 3) != 0 || ((uintptr_t)d_table & 15) != 0)
+        return bm_launch_rows_ex(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0);
+    if ((s = bm_launch_rows_gen(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0, nullptr, 0, nullptr, nullptr,
+                                true)) != BM_OK)
+        return s;
+    const SumArgs sa{d_table, ld, n, ctx->ov, A.has_self && B.has_self, A.self_w, B.self_w, ctx->pi};
+    const int64_t T = (n + kTile) / kTile;
+    tile_sum_kernel<<<(unsigned)(T * (T + 1) / 2), 256, 0, ctx->stream>>>(sa);
+    BM_LAUNCH_CHECK(ctx, "tile_sum_kernel");
+    if (A.m_out > 0) {
+        const unsigned blocks = (unsigned)std::min<int64_t>((A.m_out + 2047) / 2048, (int64_t)ctx->num_sms * 8);
+        repair_kernel<<<blocks, 256, 0, ctx->stream>>>(gview(A), hview(B), ctx->pi, n, d_table, ld);
+        BM_LAUNCH_CHECK(ctx, "repair_kernel");
+    }
+    return BM_OK;
 }
 
 extern "C" bm_status bm_table_refresh_dev(bm_ctx* ctx, int32_t* d_table, int64_t ld, const int32_t* d_rows,
