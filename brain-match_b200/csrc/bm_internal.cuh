@@ -371,6 +371,25 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
 // (d_tab 16-byte aligned, tab_ld a multiple of 4 and at least n + 1): half the
 // scatter of a delta row, whose other half is G_v(pi u).
 bm_status bm_launch_apply(bm_ctx* ctx, const int32_t* d_pairs, int32_t k);
+// One-sided gains of all rows and their transpose, kept through a search
+// (bm_gain.cu); held by one call and freed with it.
+struct BmGains {
+    void* mem = nullptr;
+    int32_t* T = nullptr;     // [u * ld + v]: gain of u at the image of v
+    int32_t* H = nullptr;     // [hrow[v] * ld + u]: the same
+    int64_t ld = 0;
+    int32_t* hrow = nullptr;
+    uint2* list_w = nullptr;  // scratch of updates
+    int32_t* list_idx = nullptr;
+    int32_t* list_n = nullptr;
+    bool held() const { return mem != nullptr; }
+};
+void bm_gains_free(BmGains* g);
+bool bm_gains_possible(bm_ctx* ctx);
+bool bm_gains_pay(const bm_ctx* ctx, int64_t pass_accepts, int32_t passes);
+bm_status bm_gains_build(bm_ctx* ctx, BmGains* g, bool* ok);
+bm_status bm_gains_rows_best(bm_ctx* ctx, const BmGains& g, const int32_t* d_rows, int32_t nrows, bm_row_result* d_res);
+bm_status bm_gains_apply(bm_ctx* ctx, const BmGains& g, const int32_t* d_pairs, int32_t k);
 bm_status bm_rows_smem_check(bm_ctx* ctx);
 bm_status bm_launch_kset(bm_ctx* ctx, int32_t k, const int32_t* d_sets, int64_t nsets, long long* d_best,
                          int32_t* d_perm, long long* d_all, int32_t* d_status);

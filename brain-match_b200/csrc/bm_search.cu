@@ -16,7 +16,14 @@
 // no A edge between two chosen swaps, the independence rule of
 // src/independent-hungarian/hungarianSubset.c:657-740) applied in one launch.
 // Independent swaps do not change each other's deltas, so the tracked score
-// stays exact.
+// stays exact.  Two things are done ahead of need there, without changing a
+// result.  Several batches are evaluated in one launch while batches accept
+// nothing (doubling, halved by an accept); they are consumed in order, and what
+// follows an accept is discarded and evaluated again.  And once a pass accepts
+// few swaps, the gains of all rows are kept in tables (bm_gain.cu), so that a
+// batch is read instead of scattered.  The full-scale search from the greedy
+// start (60 passes, the last 50 with 146 accepts and fewer) took 735-755 ms with
+// one scattered batch a launch and takes 300-330 ms so.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -216,62 +223,102 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
     int32_t R = rows_per_batch > 0 ? rows_per_batch : 2 * ctx->num_sms;
     R = std::min(R, nr);
     SchedBufs b;
-    if ((s = sched_bufs(ctx, R, &b)) != BM_OK) return s;
+    if ((s = sched_bufs(ctx, nr, &b)) != BM_OK) return s;
     if ((s = bm_rows_refresh_work(ctx)) != BM_OK) return s;
     std::vector<int32_t> cand;
     BmMarks mk;
+    struct GainsGuard {
+        BmGains g;
+        ~GainsGuard() { bm_gains_free(&g); }
+    } gains;
+    const bool may_gain = bm_gains_possible(ctx);
+    bool no_room = false;
     const auto t0 = clk::now();
     int32_t pos = prog->next_row_pos;
     if (pos < 0 || pos >= nr) pos = 0;
     bool pass_full = (pos == 0);
     int64_t pass_accepts = 0, accepts0 = prog->accepts;
+    int32_t ahead = 1;  // batches of a launch
     prog->converged = 0;
     bm_status ret = BM_OK;
-    for (;;) {
-        if (max_accepts >= 0 && prog->accepts - accepts0 >= max_accepts) break;
-        if (target_score > 0 && ctx->score >= target_score) break;
-        if (time_budget_s > 0 && secs_since(t0) >= time_budget_s) { ret = BM_TIMEOUT; break; }
-        const int32_t k = std::min(R, nr - pos);
-        for (int32_t i = 0; i < k; i++) b.h_rows[i] = order[(size_t)(pos + i)];
-        if ((s = eval_rows(ctx, b, k, false)) != BM_OK) return s;
-        prog->launches++;
-        prog->evaluated += (int64_t)k * (n - 1);
-        cand.clear();
-        for (int32_t i = 0; i < k; i++)
-            if (b.h_res[i].best_delta > 0) cand.push_back(i);
-        std::sort(cand.begin(), cand.end(), [&](int32_t x, int32_t y) {
-            if (b.h_res[x].best_delta != b.h_res[y].best_delta) return b.h_res[x].best_delta > b.h_res[y].best_delta;
-            return x < y;
-        });
-        mk.reset(n);
+    auto stop = [&]() -> bool {
+        if (max_accepts >= 0 && prog->accepts - accepts0 >= max_accepts) return true;
+        if (target_score > 0 && ctx->score >= target_score) return true;
+        if (time_budget_s > 0 && secs_since(t0) >= time_budget_s) { ret = BM_TIMEOUT; return true; }
+        return false;
+    };
+    bool done = false;
+    while (!done) {
+        if (stop()) break;
+        const int32_t held = (int32_t)std::min<int64_t>((int64_t)R * ahead, nr - pos);  // rows of the launch
+        for (int32_t i = 0; i < held; i++) b.h_rows[i] = order[(size_t)(pos + i)];
+        if (gains.g.held()) {
+            BM_CUDA(ctx, cudaMemcpyAsync(b.d_rows, b.h_rows, sizeof(int32_t) * held, cudaMemcpyHostToDevice, ctx->stream));
+            if ((s = bm_gains_rows_best(ctx, gains.g, b.d_rows, held, b.d_res)) != BM_OK) return s;
+            BM_CUDA(ctx, cudaMemcpyAsync(b.h_res, b.d_res, sizeof(bm_row_result) * held, cudaMemcpyDeviceToHost, ctx->stream));
+            BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+        } else if ((s = eval_rows(ctx, b, held, false)) != BM_OK) {
+            return s;
+        }
         int32_t na = 0;
-        int64_t gain = 0;
-        for (int32_t i : cand) {
-            const int32_t u = b.h_res[i].row, v = b.h_res[i].best;
-            if (mk.marked(u) || mk.marked(v)) continue;
-            mk.mark_closed(ctx, u);
-            mk.mark_closed(ctx, v);
-            b.h_pairs[2 * na] = u;
-            b.h_pairs[2 * na + 1] = v;
-            gain += b.h_res[i].best_delta;
-            na++;
+        for (int32_t r0 = 0; r0 < held && na == 0 && !done; r0 += R) {
+            if (r0 > 0 && stop()) { done = true; break; }
+            const int32_t k = std::min(R, held - r0);
+            const bm_row_result* res = b.h_res + r0;
+            prog->launches++;
+            prog->evaluated += (int64_t)k * (n - 1);
+            cand.clear();
+            for (int32_t i = 0; i < k; i++)
+                if (res[i].best_delta > 0) cand.push_back(i);
+            std::sort(cand.begin(), cand.end(), [&](int32_t x, int32_t y) {
+                if (res[x].best_delta != res[y].best_delta) return res[x].best_delta > res[y].best_delta;
+                return x < y;
+            });
+            mk.reset(n);
+            int64_t gain = 0;
+            for (int32_t i : cand) {
+                const int32_t u = res[i].row, v = res[i].best;
+                if (mk.marked(u) || mk.marked(v)) continue;
+                mk.mark_closed(ctx, u);
+                mk.mark_closed(ctx, v);
+                b.h_pairs[2 * na] = u;
+                b.h_pairs[2 * na + 1] = v;
+                gain += res[i].best_delta;
+                na++;
+            }
+            if (na > 0) {
+                if (gains.g.held()) {
+                    BM_CUDA(ctx, cudaMemcpyAsync(b.d_pairs, b.h_pairs, sizeof(int32_t) * 2 * na, cudaMemcpyHostToDevice,
+                                                 ctx->stream));
+                    if ((s = bm_gains_apply(ctx, gains.g, b.d_pairs, na)) != BM_OK) return s;
+                } else if ((s = apply_pairs(ctx, b, na)) != BM_OK) {
+                    return s;
+                }
+                ctx->score += gain;
+                prog->accepts += na;
+                pass_accepts += na;
+            }
+            prog->rows_done += k;
+            pos += k;
+            if (pos >= nr) {
+                pos = 0;
+                if (pass_full) prog->sweeps++;
+                if (pass_full && pass_accepts == 0) {
+                    prog->converged = 1;
+                    done = true;
+                } else if (max_sweeps >= 0 && prog->sweeps >= max_sweeps) {
+                    done = true;
+                } else if (pass_full && may_gain && !no_room && !gains.g.held() &&
+                           bm_gains_pay(ctx, pass_accepts, max_sweeps < 0 ? -1 : max_sweeps - prog->sweeps)) {
+                    bool ok = false;
+                    if ((s = bm_gains_build(ctx, &gains.g, &ok)) != BM_OK) return s;
+                    no_room = !ok;
+                }
+                pass_full = true;
+                pass_accepts = 0;
+            }
         }
-        if (na > 0) {
-            if ((s = apply_pairs(ctx, b, na)) != BM_OK) return s;
-            ctx->score += gain;
-            prog->accepts += na;
-            pass_accepts += na;
-        }
-        prog->rows_done += k;
-        pos += k;
-        if (pos >= nr) {
-            pos = 0;
-            if (pass_full) prog->sweeps++;
-            if (pass_full && pass_accepts == 0) { prog->converged = 1; break; }
-            pass_full = true;
-            pass_accepts = 0;
-            if (max_sweeps >= 0 && prog->sweeps >= max_sweeps) break;
-        }
+        ahead = na > 0 ? std::max(1, ahead / 2) : (int32_t)std::min<int64_t>(2 * (int64_t)ahead, (nr + R - 1) / R);
     }
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     prog->next_row_pos = pos;
