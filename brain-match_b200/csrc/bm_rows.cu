@@ -165,6 +165,22 @@ __device__ __forceinline__ bm_row_result row_result(int32_t u, const Partial& t)
     return out;
 }
 
+// A row's result.  In host memory that the caller polls, the row id is written
+// last, after a system-scope fence.
+__device__ __forceinline__ void put_result(bm_row_result* d, const bm_row_result& o, int host_res) {
+    if (host_res) {
+        d->first_pos = o.first_pos;
+        d->first_delta = o.first_delta;
+        d->best = o.best;
+        d->best_delta = o.best_delta;
+        d->npos = o.npos;
+        __threadfence_system();
+        *reinterpret_cast<volatile int32_t*>(&d->row) = o.row;
+    } else {
+        *d = o;
+    }
+}
+
 // REFCPU: reference-delta semantics; GAINS: one-sided sums of whole rows into
 // the table (separate instantiations, so the exact one carries none of their
 // code or registers)
@@ -703,7 +719,7 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
                         better_best(c.best_v, c.best_d, pq.best_v, pq.best_d);
                         c.npos += pq.npos;
                     }
-                    a.res[r] = row_result(u, c);
+                    put_result(a.res + r, row_result(u, c), a.host_res);
                 }
             } else {
                 *cluster.map_shared_rank(parts + crank, 0) = t;
@@ -718,19 +734,7 @@ __global__ void __launch_bounds__(THREADS, 2) rows_kernel(RowArgs a) {
             better_best(t.best_v, t.best_d, parts[q].best_v, parts[q].best_d);
             t.npos += parts[q].npos;
         }
-        const bm_row_result o = row_result(u, t);
-        if (a.host_res) {
-            bm_row_result* d = a.res + r;
-            d->first_pos = o.first_pos;
-            d->first_delta = o.first_delta;
-            d->best = o.best;
-            d->best_delta = o.best_delta;
-            d->npos = o.npos;
-            __threadfence_system();
-            *reinterpret_cast<volatile int32_t*>(&d->row) = o.row;
-        } else {
-            a.res[r] = o;
-        }
+        put_result(a.res + r, row_result(u, t), a.host_res);
     }
 }
 
