@@ -304,11 +304,17 @@ __global__ void twins_hash_kernel(const uint8_t* __restrict__ keep, const int32_
 
 size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Temporary device memory of one build, one allocation.
+// Temporary device memory of one build: up to kStagedScratch in the context's
+// staging buffer, which later calls use too (a fresh allocation and its release
+// cost a new context milliseconds), above that one allocation given back at
+// the end.
+constexpr size_t kStagedScratch = (size_t)32 << 20;
+
 struct Arena {
     char* base = nullptr;
+    bool own = false;
     size_t used = 0;
-    ~Arena() { bm_cuda_free(base); }
+    ~Arena() { if (own) bm_cuda_free(base); }
     template <typename T>
     T* take(size_t count) {
         T* p = reinterpret_cast<T*>(base + used);
@@ -366,10 +372,15 @@ bm_status bm_build_graph_dev(bm_ctx* ctx, bool side_b, int32_t n, int64_t m, con
     const size_t need = al256(sizeof(BuildStats)) + al256(4 * M) * 8 + al256(M) + al256(4 * (size_t)kMaxDigits * tiles) +
                         al256(4 * kMaxDigits) + al256(4 * (size_t)tiles) * 2 + al256(4 * V) * 4 + al256(8 * V) +
                         (side_b ? 0 : 3 * al256(4 * lists)) + 4096;
-    if (bm_cuda_malloc(&A.base, need) != cudaSuccess) {
+    if (need <= kStagedScratch) {
+        BUILD_TRY(bm_stage(ctx, need));
+        A.base = (char*)ctx->stage;
+    } else if (bm_cuda_malloc(&A.base, need) != cudaSuccess) {
         cudaGetLastError();
         *rejected = true;
         return BM_OK;
+    } else {
+        A.own = true;
     }
     BuildStats* st = A.take<BuildStats>(1);
     int32_t* d_src = A.take<int32_t>(M);
