@@ -202,7 +202,9 @@ bm_status bm_hstage(bm_ctx* ctx, size_t bytes) {
     if (ctx->hstage) bm_cuda_host_free(ctx->hstage);
     ctx->hstage = nullptr;
     ctx->hstage_bytes = 0;
-    size_t sz = bytes < (1u << 20) ? (1u << 20) : bytes;
+    // pinning costs milliseconds a megabyte: a context that only asks for rows
+    // pays for 64 KB
+    size_t sz = bytes < (1u << 16) ? (1u << 16) : bytes;
     BM_CUDA(ctx, bm_cuda_host_malloc(&ctx->hstage, sz));
     ctx->hstage_bytes = sz;
     return BM_OK;

@@ -370,6 +370,9 @@ bm_status bm_launch_rows_gen(bm_ctx* ctx, const int32_t* d_rows, const int32_t* 
 // gains: the one-sided sums of whole rows, d_tab[u * tab_ld + v] = G_u(pi v)
 // (d_tab 16-byte aligned, tab_ld a multiple of 4 and at least n + 1): half the
 // scatter of a delta row, whose other half is G_v(pi u).
+// Waits until the row ids of res[0..nrows) (pinned; reset to 0 before a launch
+// with row_host_res) have all arrived; bounded, then the stream is waited for.
+bm_status bm_poll_rows(bm_ctx* ctx, const bm_row_result* res, int32_t nrows);
 bm_status bm_launch_apply(bm_ctx* ctx, const int32_t* d_pairs, int32_t k);
 // One-sided gains of all rows and their transpose, kept through a search
 // (bm_gain.cu); held by one call and freed with it.

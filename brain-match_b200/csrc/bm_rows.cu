@@ -1155,6 +1155,23 @@ extern "C" bm_status bm_delta_rows(bm_ctx* ctx, const int32_t* rows, int32_t nro
     return BM_OK;
 }
 
+bm_status bm_poll_rows(bm_ctx* ctx, const bm_row_result* res, int32_t nrows) {
+    constexpr int64_t kPolls = 20000000;  // about a second, then the stream is waited for
+    auto arrived = [&]() {
+        for (int32_t r = 0; r < nrows; r++)
+            if (*reinterpret_cast<const volatile int32_t*>(&res[r].row) == 0) return false;
+        return true;
+    };
+    for (int64_t it = 0;; it++) {
+        if (arrived()) return BM_OK;
+        // every 1024 polls: stop polling once the stream has finished or failed
+        if ((it & 1023) == 1023 && (it > kPolls || cudaStreamQuery(ctx->stream) != cudaErrorNotReady)) break;
+    }
+    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (!arrived()) return bm_fail(ctx, BM_CUDA_ERROR, "row results missing after the row launch finished");
+    return BM_OK;
+}
+
 namespace {
 
 // Whether a host-row launch of nrows rows would take a split plan (then the
@@ -1174,7 +1191,6 @@ bool split_would_apply(const bm_ctx* ctx, int32_t nrows) {
 }
 
 constexpr int32_t kRowGraphMaxRows = 4096;
-constexpr int64_t kRowPollMax = 20000000;  // result polls before waiting on the stream (about a second)
 
 // bm_rows_best without column bounds as a replayed CUDA graph: the rows are
 // copied (CPU) into pinned staging, the graph copies them in and runs the row
@@ -1209,24 +1225,7 @@ bm_status rows_best_graph(bm_ctx* ctx, const int32_t* rows, int32_t nrows, bm_ro
         std::memcpy(h_in, rows, sizeof(int32_t) * (size_t)nrows);
         for (int32_t r = 0; r < nrows; r++) h_out[r].row = 0;
         BM_CUDA(ctx, cudaGraphLaunch(G.exec, ctx->stream));
-        auto arrived = [&]() {
-            for (int32_t r = 0; r < nrows; r++)
-                if (*reinterpret_cast<volatile int32_t*>(&h_out[r].row) == 0) return false;
-            return true;
-        };
-        bool done = false;
-        for (int64_t it = 0; !done; it++) {
-            done = arrived();
-            // every 1024 polls: stop polling once the stream has finished or
-            // failed, or after about a second
-            if (!done && (it & 1023) == 1023 &&
-                (cudaStreamQuery(ctx->stream) != cudaErrorNotReady || it > (int64_t)kRowPollMax))
-                break;
-        }
-        if (!done) {
-            BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (!arrived()) return bm_fail(ctx, BM_CUDA_ERROR, "row results missing after the row graph finished");
-        }
+        if ((s = bm_poll_rows(ctx, h_out, nrows)) != BM_OK) return s;
         ctx->launches += G.launches;
         std::memcpy(out, h_out, ob);
         return BM_OK;
@@ -1280,6 +1279,30 @@ bm_status rows_best_graph(bm_ctx* ctx, const int32_t* rows, int32_t nrows, bm_ro
     return BM_OK;
 }
 
+// The calls that the graph does not take (column bounds, a split plan): one
+// copy in from pinned staging, results polled in pinned memory.  One row of the
+// 2,000-vertex pair: 37 us with pageable copies both ways and a synchronise,
+// 28 us so.
+bm_status rows_best_polled(bm_ctx* ctx, const int32_t* rows, const int32_t* col_lo, int32_t nrows, bm_row_result* out) {
+    const size_t in = sizeof(int32_t) * (size_t)nrows * (col_lo ? 2 : 1), in_al = (in + 255) & ~(size_t)255;
+    const size_t ob = sizeof(bm_row_result) * (size_t)nrows;
+    bm_status s = bm_stage(ctx, in_al);
+    if (s != BM_OK) return s;
+    if ((s = bm_hstage(ctx, in_al + ob)) != BM_OK) return s;
+    int32_t *h_in = (int32_t*)ctx->hstage, *d_in = (int32_t*)ctx->stage;
+    bm_row_result* h_out = (bm_row_result*)((char*)ctx->hstage + in_al);
+    std::memcpy(h_in, rows, sizeof(int32_t) * (size_t)nrows);
+    if (col_lo) std::memcpy(h_in + nrows, col_lo, sizeof(int32_t) * (size_t)nrows);
+    for (int32_t r = 0; r < nrows; r++) h_out[r].row = 0;
+    BM_CUDA(ctx, cudaMemcpyAsync(d_in, h_in, in, cudaMemcpyHostToDevice, ctx->stream));
+    ctx->row_host_res = true;
+    s = bm_launch_rows(ctx, d_in, col_lo ? d_in + nrows : nullptr, nrows, nullptr, h_out, h_in);
+    ctx->row_host_res = false;
+    if (s != BM_OK || (s = bm_poll_rows(ctx, h_out, nrows)) != BM_OK) return s;
+    std::memcpy(out, h_out, ob);
+    return BM_OK;
+}
+
 }  // namespace
 
 extern "C" bm_status bm_rows_best(bm_ctx* ctx, const int32_t* rows, const int32_t* col_lo, int32_t nrows,
@@ -1290,6 +1313,7 @@ extern "C" bm_status bm_rows_best(bm_ctx* ctx, const int32_t* rows, const int32_
     if (nrows == 0) return BM_OK;
     if ((s = check_rows(ctx, rows, nrows)) != BM_OK) return s;
     if (!col_lo && nrows <= kRowGraphMaxRows && !split_would_apply(ctx, nrows)) return rows_best_graph(ctx, rows, nrows, out);
+    if (nrows <= kRowGraphMaxRows) return rows_best_polled(ctx, rows, col_lo, nrows, out);
     const size_t rb = (sizeof(int32_t) * (size_t)nrows + 255) & ~(size_t)255;
     const size_t ob = sizeof(bm_row_result) * (size_t)nrows;
     if ((s = bm_stage(ctx, 2 * rb + ob)) != BM_OK) return s;

@@ -94,8 +94,6 @@ struct StepBufs {
     int32_t* cols() const { return h_in + 64 + kmax; }
 };
 
-constexpr int64_t kStepPolls = 20000000;  // about a second, then the stream is waited for
-
 bm_status step_bufs(bm_ctx* ctx, int32_t kmax, StepBufs* b) {
     const size_t in = (sizeof(int32_t) * (64 + 2 * (size_t)kmax) + 255) & ~(size_t)255;
     bm_status s = bm_stage(ctx, in);
@@ -118,18 +116,7 @@ bm_status step_rows(bm_ctx* ctx, StepBufs& b, bool swap, int32_t k) {
     s = bm_launch_rows(ctx, b.d_in + 64, b.d_in + 64 + b.kmax, k, nullptr, b.h_res, b.rows());
     ctx->row_host_res = false;
     if (s != BM_OK) return s;
-    auto arrived = [&]() {
-        for (int32_t i = 0; i < k; i++)
-            if (*reinterpret_cast<volatile int32_t*>(&b.h_res[i].row) == 0) return false;
-        return true;
-    };
-    for (int64_t it = 0;; it++) {
-        if (arrived()) return BM_OK;
-        if ((it & 1023) == 1023 && (it > kStepPolls || cudaStreamQuery(ctx->stream) != cudaErrorNotReady)) break;
-    }
-    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (!arrived()) return bm_fail(ctx, BM_CUDA_ERROR, "row results missing after the row launch finished");
-    return BM_OK;
+    return bm_poll_rows(ctx, b.h_res, k);
 }
 
 bm_status apply_pairs(bm_ctx* ctx, SchedBufs& b, int32_t k) {
