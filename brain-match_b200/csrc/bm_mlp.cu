@@ -80,8 +80,8 @@ struct bm_mlp {
     float* d_w = nullptr;      // FP32 master parameters
     float* d_m = nullptr;      // AdamW first moment
     float* d_v = nullptr;      // AdamW second moment
-    float* d_g = nullptr;      // gradient of the last batch
-    float* d_loss = nullptr;
+    float* d_g = nullptr;      // gradient of the last batch; its loss and the error flag follow it, so
+    float* d_loss = nullptr;   // that a training call clears and reads them in one piece
     float* d_tab = nullptr;    // per-vertex table [(n+1) * 12]
     float2* d_bdeg = nullptr;  // per B vertex: log1p out-degree, log1p in-degree
     unsigned char* d_img = nullptr;
@@ -1746,8 +1746,7 @@ bm_status launch_score_simt(bm_mlp* M, PairSrc P, int64_t k, float* d_out) {
 // tensor cores (backend 0, records given as features) or the SIMT kernel.
 bm_status launch_grad(bm_mlp* M, PairSrc P, const float* d_y, int64_t k) {
     bm_ctx* ctx = M->ctx;
-    BM_CUDA(ctx, cudaMemsetAsync(M->d_g, 0, sizeof(float) * (size_t)kNParams, ctx->stream));
-    BM_CUDA(ctx, cudaMemsetAsync(M->d_loss, 0, sizeof(float), ctx->stream));
+    BM_CUDA(ctx, cudaMemsetAsync(M->d_g, 0, sizeof(float) * ((size_t)kNParams + 1), ctx->stream));
     if (M->backend == 0 && (P.xin || P.xbf)) {
         if (M->img_dirty) {
             prep_image_kernel<<<64, 256, 0, ctx->stream>>>(M->d_w, M->d_img);
@@ -1780,15 +1779,15 @@ bm_status launch_adamw(bm_mlp* M, float lr, float wd) {
     return BM_OK;
 }
 
-// Scores of rows x all partners into M->d_sc (row r at r * n).
-// Scores of rows x all partners into M->d_sc (row r at r * n), or, with
-// d_cands, of rows x their S listed partners (row r at r * S).
+// Scores of rows x all partners (row r at r * n), or, with d_cands, of rows x
+// their S listed partners (row r at r * S), into d_out or, without one, into
+// M->d_sc.
 bm_status launch_row_scores(bm_mlp* M, const int32_t* d_rows, int32_t nrows, const int32_t* d_cands = nullptr,
-                            int32_t S = 0) {
+                            int32_t S = 0, float* d_out = nullptr) {
     bm_ctx* ctx = M->ctx;
     const int32_t span = d_cands ? S : M->n;
     const size_t need = (size_t)nrows * (size_t)span;
-    if (need > M->sc_cap) {
+    if (!d_out && need > M->sc_cap) {
         bm_cuda_free(M->d_sc);
         M->d_sc = nullptr;
         M->sc_cap = 0;
@@ -1798,9 +1797,10 @@ bm_status launch_row_scores(bm_mlp* M, const int32_t* d_rows, int32_t nrows, con
         }
         M->sc_cap = need;
     }
+    if (!d_out) d_out = M->d_sc;
     if (M->backend == 1) {
         PairSrc P{nullptr, nullptr, nullptr, d_rows, span, d_cands};
-        return launch_score_simt(M, P, (int64_t)nrows * span, M->d_sc);
+        return launch_score_simt(M, P, (int64_t)nrows * span, d_out);
     }
     if (M->img_dirty) {
         prep_image_kernel<<<64, 256, 0, ctx->stream>>>(M->d_w, M->d_img);
@@ -1808,7 +1808,7 @@ bm_status launch_row_scores(bm_mlp* M, const int32_t* d_rows, int32_t nrows, con
         M->img_dirty = false;
     }
     const DevGraph& B = ctx->g[1];
-    TcArgs a{M->d_img, M->d_tab, d_rows, nrows, M->n, B.out_ptr, B.out_ent, B.in_ptr, B.in_ent, ctx->pi, M->d_sc,
+    TcArgs a{M->d_img, M->d_tab, d_rows, nrows, M->n, B.out_ptr, B.out_ent, B.in_ptr, B.in_ent, ctx->pi, d_out,
              M->d_flag, ctx->wait_limit > 0 ? (long long)ctx->wait_limit : kWaitLimit, d_cands, span};
     const int grid = std::min(nrows, ctx->num_sms);
     mlp_rows_tc_kernel<<<grid, kTcThreads, tc_smem_bytes(M->n), ctx->stream>>>(a);
@@ -1833,6 +1833,23 @@ bm_status check_flag(bm_mlp* M) {
         return bm_fail(ctx, BM_TIMEOUT, "tensor-core kernel: an MMA completion wait ran out");
     }
     return BM_OK;
+}
+
+// What a training call reports: the gradient (optional), the loss and the
+// error flag in one copy out.
+bm_status read_training(bm_mlp* M, float* grads, float* loss) {
+    bm_ctx* ctx = M->ctx;
+    const size_t head = grads ? (size_t)kNParams : 0, count = head + 2;
+    bm_status s = bm_hstage(ctx, sizeof(float) * count);
+    if (s != BM_OK) return s;
+    float* h = (float*)ctx->hstage;
+    BM_CUDA(ctx, cudaMemcpyAsync(h, M->d_g + kNParams - head, sizeof(float) * count, cudaMemcpyDeviceToHost, ctx->stream));
+    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (grads) memcpy(grads, h, sizeof(float) * head);
+    if (loss) *loss = h[head];
+    int32_t f;
+    memcpy(&f, h + head + 1, sizeof f);
+    return f ? check_flag(M) : BM_OK;
 }
 
 bm_status ensure_records(bm_mlp* M, int64_t cap) {
@@ -1920,13 +1937,7 @@ bm_status fit_steps(bm_mlp* M, int32_t steps, int32_t batch, float lr, float wd,
         if (st != BM_OK) return st;
         if ((st = launch_adamw(M, lr, wd)) != BM_OK) return st;
     }
-    if (loss) {
-        float l = 0.f;
-        BM_CUDA(ctx, cudaMemcpyAsync(&l, M->d_loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-        BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        *loss = l;
-    }
-    return check_flag(M);
+    return read_training(M, nullptr, loss);
 }
 
 }  // namespace
@@ -1938,8 +1949,8 @@ extern "C" void bm_mlp_destroy(bm_mlp* M) {
     // the context may already be gone: synchronise the device, not its stream
     cudaSetDevice(M->device);
     cudaDeviceSynchronize();
-    bm_cuda_free(M->d_w); bm_cuda_free(M->d_m); bm_cuda_free(M->d_v); bm_cuda_free(M->d_g); bm_cuda_free(M->d_loss);
-    bm_cuda_free(M->d_tab); bm_cuda_free(M->d_bdeg); bm_cuda_free(M->d_img); bm_cuda_free(M->d_sc); bm_cuda_free(M->d_flag);
+    bm_cuda_free(M->d_w); bm_cuda_free(M->d_m); bm_cuda_free(M->d_v); bm_cuda_free(M->d_g);
+    bm_cuda_free(M->d_tab); bm_cuda_free(M->d_bdeg); bm_cuda_free(M->d_img); bm_cuda_free(M->d_sc);
     bm_cuda_free(M->d_rx); bm_cuda_free(M->d_ry); bm_cuda_free(M->d_bx); bm_cuda_free(M->d_by); bm_cuda_free(M->d_scr);
     delete M;
 }
@@ -1970,19 +1981,20 @@ extern "C" bm_status bm_mlp_create(bm_ctx* ctx, uint64_t seed, bm_mlp** out) {
     init(kOffW2, BM_MLP_H, BM_MLP_H, BM_MLP_H * BM_MLP_H);
     init(kOffW3, BM_MLP_H, 1, BM_MLP_H);
     const size_t pb = sizeof(float) * (size_t)kNParams;
+    const size_t gb = pb + 2 * sizeof(float);
     const size_t tb = sizeof(float) * ((size_t)ctx->n + 1) * BM_FT;
-    if (bm_cuda_malloc(&M->d_w, pb) || bm_cuda_malloc(&M->d_m, pb) || bm_cuda_malloc(&M->d_v, pb) || bm_cuda_malloc(&M->d_g, pb) ||
-        bm_cuda_malloc(&M->d_loss, 256) || bm_cuda_malloc(&M->d_tab, tb) ||
-        bm_cuda_malloc(&M->d_bdeg, sizeof(float2) * ((size_t)ctx->n + 1)) || bm_cuda_malloc(&M->d_img, kImgBytes) ||
-        bm_cuda_malloc(&M->d_flag, 256)) {
+    if (bm_cuda_malloc(&M->d_w, pb) || bm_cuda_malloc(&M->d_m, pb) || bm_cuda_malloc(&M->d_v, pb) || bm_cuda_malloc(&M->d_g, gb) ||
+        bm_cuda_malloc(&M->d_tab, tb) ||
+        bm_cuda_malloc(&M->d_bdeg, sizeof(float2) * ((size_t)ctx->n + 1)) || bm_cuda_malloc(&M->d_img, kImgBytes)) {
         cudaGetLastError();
         bm_mlp_destroy(M);
         return bm_fail(ctx, BM_OOM, "bm_mlp_create: device allocation failed");
     }
+    M->d_loss = M->d_g + kNParams;
+    M->d_flag = reinterpret_cast<int32_t*>(M->d_loss + 1);
     if (cudaMemcpy(M->d_w, w.data(), pb, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(M->d_m, 0, pb) != cudaSuccess || cudaMemset(M->d_v, 0, pb) != cudaSuccess ||
-        cudaMemset(M->d_g, 0, pb) != cudaSuccess || cudaMemset(M->d_tab, 0, tb) != cudaSuccess ||
-        cudaMemset(M->d_flag, 0, 256) != cudaSuccess || cudaMemset(M->d_loss, 0, 256) != cudaSuccess) {
+        cudaMemset(M->d_g, 0, gb) != cudaSuccess || cudaMemset(M->d_tab, 0, tb) != cudaSuccess) {
         bm_mlp_destroy(M);
         return bm_fail(ctx, BM_CUDA_ERROR, "bm_mlp_create: initialisation failed");
     }
@@ -2128,10 +2140,7 @@ extern "C" bm_status bm_mlp_score_rows_dev(bm_mlp* M, const int32_t* d_rows, int
     bm_ctx* ctx = M->ctx;
     if (nrows < 0 || (nrows > 0 && (!d_rows || !d_scores))) return bm_fail(ctx, BM_INVALID_ARG, "bad buffers");
     if (nrows == 0) return BM_OK;
-    if ((s = launch_row_scores(M, d_rows, nrows)) != BM_OK) return s;
-    BM_CUDA(ctx, cudaMemcpyAsync(d_scores, M->d_sc, sizeof(float) * (size_t)nrows * M->n, cudaMemcpyDeviceToDevice,
-                                 ctx->stream));
-    return BM_OK;
+    return launch_row_scores(M, d_rows, nrows, nullptr, 0, d_scores);
 }
 
 extern "C" bm_status bm_mlp_score_candidates(bm_mlp* M, const int32_t* rows, int32_t nrows, const int32_t* cands,
@@ -2206,12 +2215,7 @@ extern "C" bm_status bm_mlp_gradients(bm_mlp* M, const float* x, const float* y,
     BM_CUDA(ctx, cudaMemcpyAsync(d_y, y, sizeof(float) * (size_t)k, cudaMemcpyHostToDevice, ctx->stream));
     PairSrc P{d_x, nullptr, nullptr, nullptr, M->n};
     if ((s = launch_grad(M, P, d_y, k)) != BM_OK) return s;
-    BM_CUDA(ctx, cudaMemcpyAsync(grads, M->d_g, sizeof(float) * (size_t)kNParams, cudaMemcpyDeviceToHost, ctx->stream));
-    float l = 0.f;
-    BM_CUDA(ctx, cudaMemcpyAsync(&l, M->d_loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (loss) *loss = l;
-    return check_flag(M);
+    return read_training(M, grads, loss);
 }
 
 extern "C" bm_status bm_mlp_adamw_step(bm_mlp* M, const float* x, const float* y, int64_t k, float lr,
@@ -2229,11 +2233,7 @@ extern "C" bm_status bm_mlp_adamw_step(bm_mlp* M, const float* x, const float* y
     PairSrc P{d_x, nullptr, nullptr, nullptr, M->n};
     if ((s = launch_grad(M, P, d_y, k)) != BM_OK) return s;
     if ((s = launch_adamw(M, lr, weight_decay)) != BM_OK) return s;
-    float l = 0.f;
-    BM_CUDA(ctx, cudaMemcpyAsync(&l, M->d_loss, sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (loss) *loss = l;
-    return check_flag(M);
+    return read_training(M, nullptr, loss);
 }
 
 extern "C" bm_status bm_mlp_collect_rows(bm_mlp* M, const int32_t* rows, int32_t nrows, int32_t per_row, uint64_t seed,

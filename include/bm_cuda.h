@@ -494,8 +494,7 @@ bm_status bm_mlp_pair_features(bm_mlp* m, const int32_t* pairs, int64_t k, float
 bm_status bm_mlp_score_pairs(bm_mlp* m, const int32_t* pairs, int64_t k, float* scores);
 bm_status bm_mlp_score_features(bm_mlp* m, const float* x, int64_t k, float* scores);
 bm_status bm_mlp_score_rows(bm_mlp* m, const int32_t* rows, int32_t nrows, float* scores);
-/* Same on device buffers, asynchronous on the context stream (the scores are
- * produced in the model's own buffer and copied to d_scores).  A tensor-core
+/* Same on device buffers, asynchronous on the context stream.  A tensor-core
  * wait that ran out is reported by the next bm_mlp_status or host-side call. */
 bm_status bm_mlp_score_rows_dev(bm_mlp* m, const int32_t* d_rows, int32_t nrows, float* d_scores);
 /* Scores of listed partners: scores[r * S + i] for partner cands[r * S + i]
