@@ -84,6 +84,8 @@ constexpr int kSaThreads = 512;     // threads per CTA of the allocation-free en
 constexpr int kSaMaxK = 64;         // proposals per iteration, adaptive up to this
 constexpr int kSaMaxInitialK = 16;  // largest settable starting K
 constexpr int kSaItem = 128;        // list entries per work item (four per lane)
+constexpr int kSaLongItem = 32;     // entries of an item whose row is longer than kSaRowCap: one hash lookup a lane takes as
+                                    // long as a whole item's index, and an iteration waits for its slowest warp
 constexpr int kSaRowCap = 512;      // B row entries a warp stages in shared memory (longer rows: hash)
 constexpr int kSaSlots = 2048;      // slots of a warp's index of its staged row (a byte each)
 constexpr int kSaIndexed = 252;     // longest indexed row (slot values 1..252; 255: shared by two entries)
@@ -167,10 +169,12 @@ __device__ void chain_apply_block(const PairDev& P, int32_t* pi, int32_t* gpi, i
 // an empty slot.  (Rows of more than 252 entries are searched, rows longer
 // than the buffer use the hash; a slot that two entries of the row share is
 // marked and searched.)  64 chains of 100,000 steps on four pairs of 2,709 to
-// 8,192 vertices: 107 ms with the searches and the staged swap apply, 89 ms so;
-// what bounds an iteration now is the latency of its 16 warps an SM.  For an entry of u whose other end is v,
-// the direct-edge repair min(w, B(pi u, pi v)) + min(w, B(pi v, pi u)) is
-// added; the item sums meet in a per-proposal shared counter, then
+// 8,192 vertices: 107 ms with the searches and the staged swap apply, 88 ms
+// with the index, 84 ms with small items for the lists that use the hash; what
+// bounds an iteration now is the latency of its 16 warps an SM.  For an entry
+// of u whose other end is v, the direct-edge repair
+// min(w, B(pi u, pi v)) + min(w, B(pi v, pi u)) is added; the item sums meet in
+// a per-proposal shared counter, then
 //   delta = sum - S(u) - S(v) + self-loop terms.
 // The first accepted proposal in step order is applied and the rest are
 // discarded, so the chain is the one-at-a-time chain for every K.  K adapts
@@ -195,6 +199,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
     __shared__ double s_temp[kSaMaxK];
     __shared__ int32_t s_seglen[kSeg];             // entries per list
     __shared__ int32_t s_segbase[kSeg];            // offset of each list in its CSR
+    __shared__ int32_t s_segrow[2][kSeg];          // the B row [begin, end) that the list's entries look up
     __shared__ int32_t s_upre[kSeg + 1];           // unit prefix over the lists
     __shared__ uint8_t s_unit_seg[kSaUnitTable];   // unit -> list (when the units fit)
     __shared__ int32_t s_wsum[kW];
@@ -228,7 +233,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
         if (tid < nseg) {
             const int w = tid >> 2, kind = tid & 3;
             const uint64_t sidx = step + (uint64_t)w;
-            int32_t len = 0, base = 0;
+            int32_t len = 0, base = 0, rb = 0, re = 0;
             if (sidx < end) {
                 const bm_proposal pr = bm_sa_proposal(ch.key, sidx, P.n);
                 if (kind == 0) { s_prop[w] = pr; s_sum[w] = 0; }
@@ -236,13 +241,21 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                 const int32_t* ptr = (kind & 1) ? P.Ain_ptr : P.Aout_ptr;
                 base = __ldg(ptr + me);
                 len = __ldg(ptr + me + 1) - base;
+                const int32_t g = kind < 2 ? pi[pr.v] : pi[pr.u];
+                const int32_t* rptr = (kind & 1) ? P.Bin_ptr : P.Bout_ptr;
+                rb = __ldg(rptr + g);
+                re = __ldg(rptr + g + 1);
                 // what the decision needs besides the sums, off its path
                 if (kind & 1) s_ov[kind >> 1][w] = ov[me];
                 if (kind == 2) s_temp[w] = bm_sa_temperature(a.t0, a.log_ratio, sidx, a.steps);
             }
             s_seglen[tid] = len;
             s_segbase[tid] = base;
-            units = (len + kSaItem - 1) / kSaItem;
+            s_segrow[0][tid] = rb;
+            s_segrow[1][tid] = re;
+            // lists that look up a long row are cut into smaller items
+            const int32_t size = re - rb > kSaRowCap ? kSaLongItem : kSaItem;
+            units = (len + size - 1) / size;
         }
         // ---- exclusive block scan of the unit counts
         int32_t incl = units;
@@ -273,7 +286,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
         // warp's other buffer, and item i is searched, all at once
         {
             struct Stage {
-                int32_t item, w, kind, g, rb, re;  // B row [rb, re): no arithmetic on them until they are used
+                int32_t item, w, kind, g, rb, re;  // B row [rb, re)
                 uint32_t ent[kSaItem / 32];
             };
             auto fetch = [&](int32_t item, Stage& st) {
@@ -300,18 +313,18 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                 st.w = lo >> 2;
                 st.kind = lo & 3;
                 const bool out = !(st.kind & 1);
-                const int32_t e0 = (item - s_upre[lo]) * kSaItem, len = s_seglen[lo], base = s_segbase[lo];
+                st.rb = s_segrow[0][lo];
+                st.re = s_segrow[1][lo];
+                const bool whole = st.re - st.rb <= kSaRowCap;
+                const int32_t e0 = (item - s_upre[lo]) * (whole ? kSaItem : kSaLongItem), len = s_seglen[lo], base = s_segbase[lo];
                 const uint32_t* alist = out ? P.Aout_ent : P.Ain_ent;
 #pragma unroll
                 for (int k = 0; k < kSaItem / 32; k++) {
                     const int32_t off = e0 + lane + 32 * k;
-                    if (off < len) st.ent[k] = __ldg(alist + base + off);
+                    if (off < len && (whole || k == 0)) st.ent[k] = __ldg(alist + base + off);
                 }
                 const bm_proposal& pr = s_prop[st.w];
                 st.g = st.kind < 2 ? pi[pr.v] : pi[pr.u];
-                const int32_t* rptr = out ? P.Bout_ptr : P.Bin_ptr;
-                st.rb = __ldg(rptr + st.g);
-                st.re = __ldg(rptr + st.g + 1);
             };
             // B rows start on 16-byte boundaries (rows are padded to multiples of 4)
             auto copy_row = [&](const Stage& st, int buf) {
@@ -379,36 +392,11 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
                         }
                     }
                 } else {
-                    // the lane's lookups in flight together: the first group of
-                    // slots of each, then the few that it does not settle
-                    ulonglong2 s0[kSaItem / 32], s1[kSaItem / 32];
-                    const unsigned long long np1 = (unsigned long long)P.hb.np1;
+                    // an item of a long row: one entry a lane, one lookup in the hash
 #pragma unroll
-                    for (int k = 0; k < kSaItem / 32; k++) {
-                        const int32_t g = out ? cur.g : gx4[k], h = out ? gx4[k] : cur.g;
-                        const unsigned long long key = (unsigned long long)g * np1 + (unsigned long long)h;
-                        const ulonglong2* p =
-                            reinterpret_cast<const ulonglong2*>(P.hb.tab + (bm_hash_slot0(key, P.hb.log2) & ~3ull));
-                        s0[k] = cur.ent[k] ? __ldg(p) : make_ulonglong2(0, 0);
-                        s1[k] = cur.ent[k] ? __ldg(p + 1) : make_ulonglong2(0, 0);
-                    }
-#pragma unroll
-                    for (int k = 0; k < kSaItem / 32; k++) {
-                        wb4[k] = 0;
-                        if (cur.ent[k] == 0) continue;
-                        const int32_t g = out ? cur.g : gx4[k], h = out ? gx4[k] : cur.g;
-                        const unsigned long long key = (unsigned long long)g * np1 + (unsigned long long)h;
-                        const int from = (int)(bm_hash_slot0(key, P.hb.log2) & 3ull);
-                        const unsigned long long v[4] = {s0[k].x, s0[k].y, s1[k].x, s1[k].y};
-                        bool settled = false;
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            if (q < from || settled) continue;
-                            if (v[q] == BM_HASH_EMPTY) settled = true;
-                            else if ((v[q] >> 16) == key) { wb4[k] = (int32_t)(v[q] & 0xFFFFull); settled = true; }
-                        }
-                        if (!settled) wb4[k] = bm_hash_get(P.hb, g, h);
-                    }
+                    for (int k = 0; k < kSaItem / 32; k++) wb4[k] = 0;
+                    if (cur.ent[0])
+                        wb4[0] = out ? bm_hash_get(P.hb, cur.g, gx4[0]) : bm_hash_get(P.hb, gx4[0], cur.g);
                 }
 #pragma unroll
                 for (int k = 0; k < kSaItem / 32; k++) {
