@@ -16,23 +16,27 @@
 //
 // Kernels: reach2_kernel gives each vertex to one CTA (taken from a counter,
 // so hubs do not hold up a static share), which marks 2-hop targets in an
-// n-bit shared-memory bitmap and counts them with popc.
+// n-bit shared-memory bitmap and counts them with popc.  Neighbours with more
+// than n / 64 neighbours of their own (at least 64) have their list as a row of
+// n bits in memory, and the CTA ORs those rows, 16 bytes a thread, in
+// registers: a word of 32 bits takes about 0.6 of the time of one scattered
+// bit, and a list of n / 53 neighbours breaks even.  Bits alone took 4.5 ms a
+// graph at 18,524 vertices and 3,000,000 edges (2 x 2.4e9 targets), with the
+// rows 1.5 ms (lines at n / 32 and n / 128 were not better).
 //
-// greedy_kernel is one CTA whose 32 warps hold 32 consecutive A vertices.  Each
-// warp finds its vertex's nearest unmatched B vertex; then the vertices are
-// committed in order up to the first whose choice an earlier one of the 32 has
-// taken (a choice that is still free is still the nearest: matching others
-// only removes candidates), and only warps with a new vertex or a taken choice
-// search again.  A search starts where B's feature sum equals the vertex's and
-// goes outwards both ways: the L1 distance is at least the difference of the
-// sums, so a side ends where that difference exceeds the best distance.  The
-// unmatched vertices are kept dense (compacted every 1,024 commits).  A
-// block-wide argmin over all of B per A vertex took 131 ms at full scale;
-// this one takes 22 ms.
+// The greedy step goes in rounds of kRound A vertices.  shortlist_kernel, a
+// warp a vertex over the whole device, lists the kList nearest of the B
+// vertices that are left; then one warp of commit_kernel goes through the
+// round's vertices and gives each the first on its list that is still free (the
+// nearest: all that are not listed are further).  A vertex whose list is
+// used up is searched for then.  Searches start where B's feature sum
+// equals the vertex's and go outwards both ways: the L1 distance is at least
+// the difference of the sums, so a side ends where that difference exceeds the
+// distance to beat.  The unmatched vertices are kept dense, compacted after
+// each round.  At 18,524 vertices a block-wide argmin over all of B per A vertex
+// took 131 ms, searches by the committing CTA alone 22 ms, this takes 5.8 ms.
 #include <algorithm>
 #include <climits>
-#include <numeric>
-#include <vector>
 
 #include "bm_internal.cuh"
 
@@ -40,18 +44,27 @@ namespace {
 
 constexpr int kReachThreads = 256;
 constexpr int kGreedyThreads = 1024;
+constexpr int kListThreads = 128;
+constexpr int kRound = 256;   // A vertices between compactions of what is left of B
+constexpr int kList = 64;     // shortlist entries: two a lane; one vertex in 80 uses all of them up (rounds of 1,024: one in 25)
+
+constexpr int kReachRows = 512;  // bit rows of a stretch
 
 struct Adj {
-    const int32_t* ptr;  // n+2
-    const int32_t* idx;  // neighbour ids
+    const int32_t* ptr;   // n+2
+    const int32_t* idx;   // neighbour ids: [ptr, hend) those with a bit row, [hend, next ptr) the others
+    const int32_t* hend;  // n+1
+    const int32_t* row;   // a vertex's bit row, -1: none
+    const uint4* rows;    // n + 1 bits in 16-byte words each
 };
 
-__global__ void __launch_bounds__(kReachThreads) reach2_kernel(Adj out, Adj in, int32_t n, int* next,
+__global__ void __launch_bounds__(kReachThreads) reach2_kernel(Adj out, Adj in, int32_t n, int copies, int* next,
                                                                int4* __restrict__ feat) {
-    extern __shared__ uint32_t bits[];
+    extern __shared__ __align__(16) uint32_t bits[];
     __shared__ int s_v;
     __shared__ int s_cnt;
-    const uint32_t nw = (uint32_t)(n + 32) / 32u;
+    __shared__ int32_t s_row[kReachRows];
+    const int32_t groups = (n + 128) / 128;  // 16-byte words of n + 1 bits
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = kReachThreads / 32;
     for (;;) {
         if (tid == 0) s_v = atomicAdd(next, 1) + 1;
@@ -61,11 +74,35 @@ __global__ void __launch_bounds__(kReachThreads) reach2_kernel(Adj out, Adj in, 
         int counts[2];
         for (int dir = 0; dir < 2; dir++) {
             const Adj a = dir == 0 ? out : in;
-            for (uint32_t i = tid; i < nw; i += kReachThreads) bits[i] = 0u;
+            const int32_t j0 = a.ptr[v], jh = a.hend[v], j1 = a.ptr[v + 1];
+            for (int32_t i = tid; i < groups; i += kReachThreads) reinterpret_cast<uint4*>(bits)[i] = make_uint4(0, 0, 0, 0);
             if (tid == 0) s_cnt = 0;
+            // neighbours with a bit row, in stretches: each thread ORs its words of them
+            for (int32_t c0 = j0; c0 < jh; c0 += kReachRows) {
+                const int32_t nr = min(kReachRows, jh - c0);
+                for (int32_t j = tid; j < nr; j += kReachThreads) s_row[j] = a.row[a.idx[c0 + j]];
+                __syncthreads();
+                for (int32_t q = tid; q < groups * copies; q += kReachThreads) {
+                    const int32_t g = q % groups;
+                    uint4 acc = make_uint4(0, 0, 0, 0);
+#pragma unroll 8
+                    for (int32_t j = q / groups; j < nr; j += copies) {
+                        const uint4 r = __ldg(a.rows + (size_t)s_row[j] * groups + g);
+                        acc.x |= r.x;
+                        acc.y |= r.y;
+                        acc.z |= r.z;
+                        acc.w |= r.w;
+                    }
+                    if (acc.x) atomicOr(&bits[4 * g], acc.x);
+                    if (acc.y) atomicOr(&bits[4 * g + 1], acc.y);
+                    if (acc.z) atomicOr(&bits[4 * g + 2], acc.z);
+                    if (acc.w) atomicOr(&bits[4 * g + 3], acc.w);
+                }
+                __syncthreads();
+            }
             __syncthreads();
-            // warps take the first-step neighbours x, lanes stream x's list
-            for (int32_t j = a.ptr[v] + warp; j < a.ptr[v + 1]; j += nwarps) {
+            // the others: warps take the neighbours x, lanes stream x's list
+            for (int32_t j = jh + warp; j < j1; j += nwarps) {
                 const int32_t x = a.idx[j];
                 for (int32_t k = a.ptr[x] + lane; k < a.ptr[x + 1]; k += 32) {
                     const int32_t y = a.idx[k];
@@ -74,7 +111,7 @@ __global__ void __launch_bounds__(kReachThreads) reach2_kernel(Adj out, Adj in, 
             }
             __syncthreads();
             int c = 0;
-            for (uint32_t i = tid; i < nw; i += kReachThreads) c += __popc(bits[i]);
+            for (int32_t i = tid; i < 4 * groups; i += kReachThreads) c += __popc(bits[i]);
             for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
             if (lane == 0) atomicAdd(&s_cnt, c);
             __syncthreads();
@@ -93,15 +130,9 @@ __device__ __forceinline__ long long l1(const int4& a, const int4& b) {
 
 __device__ __forceinline__ long long total(const int4& f) { return (long long)f.x + f.y + f.z + f.w; }
 
-// The nearest unmatched B vertex of one A vertex, by a warp: the smallest key
-// = distance << 17 | sorted position, so ties go to the first position
-// (n <= 131071 < 2^17; distances stay below 2^46).  cf, cpos: the `len`
-// candidates left at the last compaction by descending sum; `used`: bits of
-// the positions matched since.
-__device__ unsigned long long nearest(const int4& f, const int4* cf, const int32_t* cpos, int32_t len,
-                                      const uint32_t* used, int lane) {
-    const long long ta = total(f);
-    // the first candidate whose sum is at most ta: 32 probes a step
+// The first candidate whose sum is at most ta (len: none), by a warp: 32
+// probes a step.
+__device__ __forceinline__ int32_t first_at_most(long long ta, const int4* cf, int32_t len, int lane) {
     int32_t lo = 0, hi = len;
     while (hi > lo) {
         const int32_t w = hi - lo, probe = lo + (int32_t)((long long)w * lane / 32);
@@ -112,7 +143,18 @@ __device__ unsigned long long nearest(const int4& f, const int4* cf, const int32
         hi = c == 32 ? hi : lo + (int32_t)((long long)w * c / 32);
         lo = nlo;
     }
-    int32_t r = lo, l = lo - 1;
+    return lo;
+}
+
+// The nearest unmatched B vertex of one A vertex, by a warp: the smallest key
+// = distance << 17 | sorted position, so ties go to the first position
+// (n <= 131071 < 2^17; distances stay below 2^46).  cf, cpos: the `len`
+// candidates left at the last compaction by descending sum; `used`: the
+// positions matched since.
+__device__ unsigned long long nearest(const int4& f, const int4* cf, const int32_t* cpos, int32_t len,
+                                      const uint8_t* used, int lane) {
+    const long long ta = total(f);
+    int32_t r = first_at_most(ta, cf, len, lane), l = r - 1;
     unsigned long long best = ~0ull;
     bool go_r = r < len, go_l = l >= 0;
     while (go_r || go_l) {
@@ -123,7 +165,7 @@ __device__ unsigned long long nearest(const int4& f, const int4* cf, const int32
                 const int4 b = cf[j];
                 const int32_t p = cpos[j];
                 const unsigned long long key = ((unsigned long long)l1(f, b) << 17) | (unsigned long long)p;
-                if (key < best && !((used[p >> 5] >> (p & 31)) & 1u)) best = key;
+                if (key < best && !used[p]) best = key;
             }
         }
         r += 64;
@@ -139,86 +181,220 @@ __device__ unsigned long long nearest(const int4& f, const int4* cf, const int32
     return best;
 }
 
-constexpr int kGreedyCompact = 1024;  // commits between compactions
+using Key = unsigned long long;
 
-// fa, ida: A vertices in sorted order (features, ids); fb, idb: the same for
-// B.  pi[ida[i]] = idb[j] for the position j chosen at step i.  cf, cpos:
-// scratch of n entries each.
-__global__ void __launch_bounds__(kGreedyThreads) greedy_kernel(const int4* __restrict__ fa,
-                                                                const int32_t* __restrict__ ida,
-                                                                const int4* __restrict__ fb,
-                                                                const int32_t* __restrict__ idb, int32_t n, int4* cf,
-                                                                int32_t* cpos, int32_t* __restrict__ pi) {
-    extern __shared__ uint32_t used[];
-    __shared__ unsigned long long s_key[32];
-    __shared__ int32_t s_new[32];  // the slot's vertex needs a search
-    __shared__ int32_t s_head, s_wsum[32];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t nw = (uint32_t)(n + 31) / 32u;
-    for (uint32_t i = tid; i < nw; i += kGreedyThreads) used[i] = 0u;
-    for (int32_t j = tid; j < n; j += kGreedyThreads) { cf[j] = fb[j]; cpos[j] = j; }
-    if (tid < 32) s_new[tid] = 1;
-    __syncthreads();
-    int32_t head = 0, len = n, compacted = 0;
-    while (head < n) {
-        const int32_t i = head + ((warp - head) & 31);  // vertex i lives in slot i mod 32
-        if (i < n && s_new[warp]) {
-            const unsigned long long best = nearest(fa[i], cf, cpos, len, used, lane);
-            if (lane == 0) s_key[warp] = best;
+__device__ __forceinline__ void order(Key& a, Key& b) {
+    const Key lo = a < b ? a : b;
+    b = a < b ? b : a;
+    a = lo;
+}
+
+// One step of a bitonic network over a warp's lanes.
+__device__ __forceinline__ void lane_step(Key& k, int lane, int stride, bool up) {
+    const Key o = __shfl_xor_sync(0xffffffffu, k, stride);
+    k = (((lane & stride) == 0) == up) == (o < k) ? o : k;
+}
+
+// Keys of 64 elements, element 32 r + lane in register r: those of (p0, p1) in
+// any order and the sorted (k0, k1) give the sorted 64 smallest in (k0, k1).
+__device__ void merge64(Key& k0, Key& k1, Key p0, Key p1, int lane) {
+#pragma unroll
+    for (int size = 2; size <= 32; size *= 2)
+#pragma unroll
+        for (int stride = size / 2; stride > 0; stride /= 2) {
+            lane_step(p0, lane, stride, (lane & size) == 0);              // lane < 32: the 32-sort ascends,
+            lane_step(p1, lane, stride, size < 32 && (lane & size) == 0);  // the second one descends
         }
-        __syncthreads();
-        if (warp == 0) {
-            const int32_t v = head + lane, slot = v & 31;
-            const int32_t j = v < n ? (int32_t)(s_key[slot] & 0x1FFFFull) : -1 - lane;
-            const unsigned same = __match_any_sync(0xffffffffu, j);
-            const unsigned clash = __ballot_sync(0xffffffffu, v >= n || (same & ((1u << lane) - 1u)) != 0u);
-            const int done = clash ? __ffs(clash) - 1 : 32;
-            if (lane < done) {
-                atomicOr(&used[j >> 5], 1u << (j & 31));
-                pi[ida[v]] = idb[j];
-            }
-            __syncwarp();
-            s_new[slot] = lane < done || (v < n && ((used[j >> 5] >> (j & 31)) & 1u));
-            if (lane == 0) s_head = head + done;
-        }
-        __syncthreads();
-        head = s_head;
-        if (head - compacted >= kGreedyCompact) {  // drop the matched candidates, in order
-            compacted = head;
-            int32_t base = 0;
-            for (int32_t j0 = 0; j0 < len; j0 += kGreedyThreads) {
-                const int32_t j = j0 + tid;
-                int4 f = make_int4(0, 0, 0, 0);
-                int32_t p = 0;
-                bool keep = false;
-                if (j < len) {
-                    f = cf[j];
-                    p = cpos[j];
-                    keep = !((used[p >> 5] >> (p & 31)) & 1u);
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, keep);
-                if (lane == 0) s_wsum[warp] = __popc(m);
-                __syncthreads();  // everything of this stretch is read
-                int32_t before = base, all = 0;
-                for (int w = 0; w < 32; w++) {
-                    if (w < warp) before += s_wsum[w];
-                    all += s_wsum[w];
-                }
-                if (keep) {
-                    const int32_t at = before + __popc(m & ((1u << lane) - 1u));
-                    cf[at] = f;
-                    cpos[at] = p;
-                }
-                base += all;
-                __syncthreads();
-            }
-            len = base;
-        }
+    order(p0, p1);
+#pragma unroll
+    for (int stride = 16; stride > 0; stride /= 2) {
+        lane_step(p0, lane, stride, true);
+        lane_step(p1, lane, stride, true);
+    }
+    const Key q0 = __shfl_sync(0xffffffffu, p1, 31 - lane), q1 = __shfl_sync(0xffffffffu, p0, 31 - lane);
+    k0 = q0 < k0 ? q0 : k0;
+    k1 = q1 < k1 ? q1 : k1;
+    order(k0, k1);
+#pragma unroll
+    for (int stride = 16; stride > 0; stride /= 2) {
+        lane_step(k0, lane, stride, true);
+        lane_step(k1, lane, stride, true);
     }
 }
 
-// Plain adjacency (ids only, any order within a list: the features are counts)
-// of both directions of an edge list.
+// list[64 i ..]: the kList smallest keys of A vertex head + i over the
+// candidates, ascending, then ~0.  A warp scans outwards from its start and
+// holds the list in registers; candidates below its last key wait in shared
+// memory until there are more than 32.
+__global__ void __launch_bounds__(kListThreads) shortlist_kernel(const int4* __restrict__ fa, int32_t head, int32_t count,
+                                                                 const int4* __restrict__ cf,
+                                                                 const int32_t* __restrict__ cpos,
+                                                                 const int32_t* __restrict__ d_len, Key* __restrict__ list) {
+    __shared__ Key s_wait[kListThreads / 32][64];
+    const int lane = threadIdx.x & 31;
+    const int32_t i = blockIdx.x * (kListThreads / 32) + (threadIdx.x >> 5);
+    if (i >= count) return;
+    Key* wait = s_wait[threadIdx.x >> 5];
+    const int4 f = fa[head + i];
+    const long long ta = total(f);
+    const int32_t len = *d_len;
+    int32_t r = first_at_most(ta, cf, len, lane), l = r - 1;
+    Key k0 = ~0ull, k1 = ~0ull, last = ~0ull;
+    int waiting = 0;
+    bool go_r = r < len, go_l = l >= 0;
+    while (go_r || go_l) {
+        Key key[2] = {~0ull, ~0ull};
+        long long edge[2] = {0, 0};  // the sum of the last candidate of this step on either side
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const int32_t j = s ? l - lane : r + lane;
+            if (s ? go_l && j >= 0 : go_r && j < len) {
+                const int4 b = cf[j];
+                key[s] = ((Key)l1(f, b) << 17) | (Key)cpos[j];
+                edge[s] = total(b);
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            const unsigned m = __ballot_sync(0xffffffffu, key[s] < last);
+            if (key[s] < last) wait[waiting + __popc(m & ((1u << lane) - 1u))] = key[s];
+            waiting += __popc(m);
+            __syncwarp();
+            if (waiting > 32) {
+                merge64(k0, k1, wait[lane], lane + 32 < waiting ? wait[lane + 32] : ~0ull, lane);
+                last = __shfl_sync(0xffffffffu, k1, 31);
+                waiting = 0;
+                __syncwarp();
+            }
+        }
+        r += 32;
+        l -= 32;
+        const long long d = last == ~0ull ? LLONG_MAX : (long long)(last >> 17);
+        const long long er = __shfl_sync(0xffffffffu, edge[0], 31), el = __shfl_sync(0xffffffffu, edge[1], 31);
+        go_r = go_r && r < len && ta - er <= d;
+        go_l = go_l && l >= 0 && el - ta <= d;
+    }
+    if (waiting > 0) merge64(k0, k1, lane < waiting ? wait[lane] : ~0ull, ~0ull, lane);
+    list[(size_t)kList * i + lane] = k0;
+    list[(size_t)kList * i + 32 + lane] = k1;
+}
+
+// Commits A vertices [first, end) (features and ids in sorted order: fa, ida).
+// pi[ida[i]] = idb[j] for the position j chosen at step i.  cf, cpos, *d_len:
+// what is left of B, before and after.  One warp goes through the vertices (a
+// shared-memory read, a vote and a store a vertex are the chain: 0.1 us); the block's
+// others load the lists and drop the matched candidates.
+__global__ void __launch_bounds__(kGreedyThreads) commit_kernel(const int4* __restrict__ fa,
+                                                                const int32_t* __restrict__ ida,
+                                                                const int32_t* __restrict__ idb, int32_t n, int32_t first,
+                                                                int32_t end, const Key* __restrict__ list, int4* cf,
+                                                                int32_t* cpos, int32_t* d_len, int32_t* __restrict__ pi) {
+    extern __shared__ __align__(16) uint8_t s_dyn[];
+    int32_t* s_list = reinterpret_cast<int32_t*>(s_dyn);     // positions, n: none
+    uint8_t* used = s_dyn + sizeof(int32_t) * kRound * kList;  // positions matched in this round, and n
+    __shared__ int32_t s_choice[kRound];
+    __shared__ int32_t s_wsum[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int32_t len = *d_len;
+    for (int32_t i = tid; i <= n / 16; i += kGreedyThreads) reinterpret_cast<uint4*>(used)[i] = make_uint4(0, 0, 0, 0);
+    for (int32_t k = tid; k < (end - first) * kList; k += kGreedyThreads) {
+        const Key key = list[k];
+        s_list[k] = key == ~0ull ? n : (int32_t)(key & 0x1FFFFull);
+    }
+    __syncthreads();
+    if (tid == 0) used[n] = 1;
+    if (warp == 0) {
+        __syncwarp();
+        int32_t p0 = s_list[lane], p1 = s_list[32 + lane];
+        for (int32_t i = 0; i < end - first; i++) {
+            const bool f0 = !used[p0], f1 = !used[p1];
+            const int32_t ahead = kList * min(i + 1, end - first - 1) + lane;
+            const int32_t q0 = s_list[ahead], q1 = s_list[ahead + 32];
+            const unsigned m0 = __ballot_sync(0xffffffffu, f0), m1 = __ballot_sync(0xffffffffu, f1);
+            int32_t p = m0 ? p0 : p1;
+            bool mine = lane == __ffs(m0 ? m0 : m1) - 1;
+            if (!(m0 | m1)) {
+                p = (int32_t)(nearest(fa[first + i], cf, cpos, len, used, lane) & 0x1FFFFull);
+                mine = lane == 0;
+            }
+            if (mine) {
+                used[p] = 1;
+                s_choice[i] = p;
+            }
+            __syncwarp();
+            p0 = q0;
+            p1 = q1;
+        }
+    }
+    __syncthreads();
+    for (int32_t i = first + tid; i < end; i += kGreedyThreads) pi[ida[i]] = idb[s_choice[i - first]];
+    int32_t base = 0;  // drop the matched candidates, in order
+    for (int32_t j0 = 0; j0 < len; j0 += kGreedyThreads) {
+        const int32_t j = j0 + tid;
+        int4 f = make_int4(0, 0, 0, 0);
+        int32_t p = 0;
+        bool keep = false;
+        if (j < len) {
+            f = cf[j];
+            p = cpos[j];
+            keep = !used[p];
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (lane == 0) s_wsum[warp] = __popc(m);
+        __syncthreads();  // everything of this stretch is read
+        int32_t before = base, all = 0;
+        for (int w = 0; w < 32; w++) {
+            if (w < warp) before += s_wsum[w];
+            all += s_wsum[w];
+        }
+        if (keep) {
+            const int32_t at = before + __popc(m & ((1u << lane) - 1u));
+            cf[at] = f;
+            cpos[at] = p;
+        }
+        base += all;
+        __syncthreads();
+    }
+    if (tid == 0) *d_len = base;
+}
+
+// Sorted positions (descending feature sum, ties by id) of both graphs'
+// vertices (blockIdx.z: 0 A, 1 B) by counting who comes before: 2 n^2
+// comparisons, and nothing goes to the host and back.  rank: 2 (n + 1), zero.
+__global__ void __launch_bounds__(256) rank_kernel(const int4* __restrict__ feat, int32_t n, int32_t* __restrict__ rank) {
+    __shared__ long long s_t[256];
+    const int4* f = feat + (size_t)blockIdx.z * (n + 1);
+    const int32_t v = 1 + blockIdx.x * 256 + threadIdx.x;
+    const long long mine = v <= n ? total(f[v]) : 0;
+    int32_t c = 0;
+    for (int32_t x0 = 1 + blockIdx.y * 256; x0 <= n; x0 += gridDim.y * 256) {
+        const int32_t y = x0 + threadIdx.x;
+        __syncthreads();
+        s_t[threadIdx.x] = y <= n ? total(f[y]) : LLONG_MIN;
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < 256; k++) c += s_t[k] > mine || (s_t[k] == mine && x0 + k < v);
+    }
+    if (v <= n && c) atomicAdd(rank + (size_t)blockIdx.z * (n + 1) + v, c);
+}
+
+// A's features and ids in sorted order; B's as the first candidates.
+__global__ void sorted_kernel(const int4* __restrict__ feat, const int32_t* __restrict__ rank, int32_t n, int4* __restrict__ fa,
+                              int32_t* __restrict__ ida, int32_t* __restrict__ idb, int4* __restrict__ cf,
+                              int32_t* __restrict__ cpos, int32_t* __restrict__ d_len) {
+    const int32_t v = 1 + blockIdx.x * blockDim.x + threadIdx.x;
+    if (v > n) return;
+    const int32_t ra = rank[v], rb = rank[n + 1 + v];
+    fa[ra] = feat[v];
+    ida[ra] = v;
+    cf[rb] = feat[n + 1 + v];
+    cpos[rb] = rb;
+    idb[rb] = v;
+    if (v == 1) *d_len = n;
+}
+
+// Plain adjacency (ids only, any order within a list but for the vertices with
+// a bit row: the features are counts) of both directions of an edge list.
 __global__ void adj_count_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int32_t n,
                                  int32_t* __restrict__ ocnt, int32_t* __restrict__ icnt, int* __restrict__ bad) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
@@ -232,16 +408,27 @@ __global__ void adj_count_kernel(const int32_t* __restrict__ src, const int32_t*
     }
 }
 
+struct Fill {  // one direction while it is built
+    int32_t* cnt;   // n+1: counts, then the front cursor of each list
+    int32_t* back;  // n+1: the back cursor
+    int32_t* ptr;   // n+2
+    int32_t* idx;
+    int32_t* row;   // n+1
+    uint32_t* rows;
+};
+
 // Exclusive sums of the counts of one direction (block 0: out, 1: in) into
-// ptr[0..n+1] and the fill cursors.
-__global__ void __launch_bounds__(1024) adj_scan_kernel(int32_t* cnt0, int32_t* cnt1, int32_t n, int32_t* ptr0, int32_t* ptr1) {
+// ptr[0..n+1] and the fill cursors; rows for vertices with more than `heavy`
+// neighbours.
+__global__ void __launch_bounds__(1024) adj_scan_kernel(Fill out, Fill in, int32_t n, int32_t heavy) {
     __shared__ int32_t wsum[32];
-    int32_t* cnt = blockIdx.x ? cnt1 : cnt0;
-    int32_t* ptr = blockIdx.x ? ptr1 : ptr0;
+    __shared__ int32_t s_rows;
+    const Fill d = blockIdx.x ? in : out;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_rows = 0;
     int32_t base = 0;
     for (int32_t v0 = 0; v0 <= n; v0 += 1024) {
-        const int32_t v = v0 + tid, c = v <= n ? cnt[v] : 0;
+        const int32_t v = v0 + tid, c = v <= n ? d.cnt[v] : 0;
         int32_t s = c;
         for (int o = 1; o < 32; o <<= 1) {
             const int32_t t = __shfl_up_sync(0xffffffffu, s, o);
@@ -255,80 +442,110 @@ __global__ void __launch_bounds__(1024) adj_scan_kernel(int32_t* cnt0, int32_t* 
             base += wsum[w];
         }
         if (v <= n) {
-            ptr[v] = before + s - c;
-            cnt[v] = before + s - c;  // becomes the fill cursor
+            d.ptr[v] = before + s - c;
+            d.cnt[v] = before + s - c;
+            d.back[v] = before + s;
+            d.row[v] = c > heavy ? atomicAdd(&s_rows, 1) : -1;
         }
         __syncthreads();
     }
-    if (tid == 0) ptr[n + 1] = base;
+    if (tid == 0) d.ptr[n + 1] = base;
 }
 
-__global__ void adj_fill_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m,
-                                int32_t* __restrict__ ocur, int32_t* __restrict__ icur, int32_t* __restrict__ oidx,
-                                int32_t* __restrict__ iidx) {
+__global__ void adj_fill_kernel(const int32_t* __restrict__ src, const int32_t* __restrict__ dst, int64_t m, int32_t n,
+                                Fill out, Fill in) {
+    const size_t words = 4 * (size_t)((n + 128) / 128);
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < m; e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t s = src[e], d = dst[e];
-        oidx[atomicAdd(ocur + s, 1)] = d;
-        iidx[atomicAdd(icur + d, 1)] = s;
+        if ((uint32_t)(s - 1) >= (uint32_t)n || (uint32_t)(d - 1) >= (uint32_t)n) continue;
+        out.idx[out.row[d] >= 0 ? atomicAdd(out.cnt + s, 1) : atomicSub(out.back + s, 1) - 1] = d;
+        in.idx[in.row[s] >= 0 ? atomicAdd(in.cnt + d, 1) : atomicSub(in.back + d, 1) - 1] = s;
+        const int32_t rs = out.row[s], rd = in.row[d];
+        if (rs >= 0) atomicOr(out.rows + rs * words + (d >> 5), 1u << (d & 31));
+        if (rd >= 0) atomicOr(in.rows + rd * words + (s >> 5), 1u << (s & 31));
     }
 }
 
-struct DevBuf {
-    std::vector<void*> p;
-    ~DevBuf() { for (void* x : p) bm_cuda_free(x); }
+// Memory of one call: a single block, cut into 256-byte aligned arrays.
+struct Arena {
+    char* mem = nullptr;
+    size_t used = 0;
+    ~Arena() { bm_cuda_free(mem); }
     template <typename T>
-    bool get(T** out, size_t count) {
-        void* d = nullptr;
-        if (bm_cuda_malloc(&d, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        p.push_back(d);
-        *out = static_cast<T*>(d);
-        return true;
+    void get(T** p, size_t count) {
+        *p = mem ? reinterpret_cast<T*>(mem + used) : nullptr;
+        used += (sizeof(T) * std::max<size_t>(count, 1) + 255) & ~(size_t)255;
     }
 };
 
-// Features (n+1 int4: in, out, reach2, canreach2) of one graph on the device;
-// *bad is set when an endpoint lies outside 1..n.
-bm_status graph_features(bm_ctx* ctx, DevBuf& mem, int32_t n, int64_t m, const int32_t* src, const int32_t* dst,
-                         std::vector<int4>& feat, bool* bad) {
+struct Work {
+    int32_t *src, *dst;
+    Fill d[2];  // out, in
+    int* misc;  // next vertex, bad endpoint, candidates left
+    int4 *feat, *fa, *cf;
+    int32_t *rank, *ida, *idb, *cpos, *pi;
+    Key* list;
+};
+
+// heavy: a list longer than this has a bit row (at most m / (heavy + 1) lists).
+void lay_out(Arena& a, Work& w, int32_t n, int64_t m, int32_t heavy) {
     const size_t M = (size_t)m, V = (size_t)n + 2;
-    int32_t *d_src, *d_dst, *d_optr, *d_oidx, *d_iptr, *d_iidx, *d_cnt;
-    int* d_next;
-    int4* d_feat;
-    if (!mem.get(&d_src, M) || !mem.get(&d_dst, M) || !mem.get(&d_cnt, 2 * V) || !mem.get(&d_optr, V) ||
-        !mem.get(&d_oidx, M) || !mem.get(&d_iptr, V) || !mem.get(&d_iidx, M) || !mem.get(&d_next, 2) ||
-        !mem.get(&d_feat, (size_t)n + 1))
-        return bm_fail(ctx, BM_OOM, "greedy matching: device allocation failed");
-    if (m > 0) {
-        BM_CUDA(ctx, cudaMemcpyAsync(d_src, src, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
-        BM_CUDA(ctx, cudaMemcpyAsync(d_dst, dst, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
+    a.used = 0;
+    a.get(&w.misc, 4);
+    a.get(&w.src, M);
+    a.get(&w.dst, M);
+    for (Fill& f : w.d) {
+        a.get(&f.cnt, V);
+        a.get(&f.back, V);
+        a.get(&f.ptr, V);
+        a.get(&f.row, V);
+        a.get(&f.idx, M);
+        a.get(&f.rows, heavy == INT32_MAX ? 1 : (M / ((size_t)heavy + 1)) * 4 * (size_t)((n + 128) / 128));
     }
-    BM_CUDA(ctx, cudaMemsetAsync(d_cnt, 0, sizeof(int32_t) * 2 * V, ctx->stream));
-    BM_CUDA(ctx, cudaMemsetAsync(d_next, 0, 2 * sizeof(int), ctx->stream));
+    a.get(&w.feat, 2 * V);
+    a.get(&w.rank, 2 * V);
+    a.get(&w.fa, V);
+    a.get(&w.cf, V);
+    a.get(&w.ida, V);
+    a.get(&w.idb, V);
+    a.get(&w.cpos, V);
+    a.get(&w.pi, V);
+    a.get(&w.list, (size_t)kRound * kList);
+}
+
+// Features (in, out, reach2, canreach2) of one graph into feat[1..n]; endpoints
+// outside 1..n set misc[1] and are left out.
+bm_status graph_features(bm_ctx* ctx, const Work& w, int32_t n, int64_t m, int32_t heavy, const int32_t* src,
+                         const int32_t* dst, int4* feat) {
+    const size_t M = (size_t)m, V = (size_t)n + 2;
+    if (m > 0) {
+        BM_CUDA(ctx, cudaMemcpyAsync(w.src, src, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
+        BM_CUDA(ctx, cudaMemcpyAsync(w.dst, dst, sizeof(int32_t) * M, cudaMemcpyHostToDevice, ctx->stream));
+    }
+    const size_t groups = (size_t)((n + 128) / 128);
+    for (const Fill& f : w.d) {
+        BM_CUDA(ctx, cudaMemsetAsync(f.cnt, 0, sizeof(int32_t) * V, ctx->stream));
+        if (heavy != INT32_MAX && m > heavy)
+            BM_CUDA(ctx, cudaMemsetAsync(f.rows, 0, M / ((size_t)heavy + 1) * groups * 16, ctx->stream));
+    }
+    BM_CUDA(ctx, cudaMemsetAsync(w.misc, 0, sizeof(int), ctx->stream));
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>((m + 255) / 256, (int64_t)ctx->num_sms * 8));
-    adj_count_kernel<<<grid, 256, 0, ctx->stream>>>(d_src, d_dst, m, n, d_cnt, d_cnt + V, d_next + 1);
+    adj_count_kernel<<<grid, 256, 0, ctx->stream>>>(w.src, w.dst, m, n, w.d[0].cnt, w.d[1].cnt, w.misc + 1);
     BM_LAUNCH_CHECK(ctx, "adj_count_kernel");
-    int h_bad = 0;
-    BM_CUDA(ctx, cudaMemcpyAsync(&h_bad, d_next + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    *bad = h_bad != 0;
-    if (*bad) return BM_OK;
-    adj_scan_kernel<<<2, 1024, 0, ctx->stream>>>(d_cnt, d_cnt + V, n, d_optr, d_iptr);
+    adj_scan_kernel<<<2, 1024, 0, ctx->stream>>>(w.d[0], w.d[1], n, heavy);
     BM_LAUNCH_CHECK(ctx, "adj_scan_kernel");
-    adj_fill_kernel<<<grid, 256, 0, ctx->stream>>>(d_src, d_dst, m, d_cnt, d_cnt + V, d_oidx, d_iidx);
+    adj_fill_kernel<<<grid, 256, 0, ctx->stream>>>(w.src, w.dst, m, n, w.d[0], w.d[1]);
     BM_LAUNCH_CHECK(ctx, "adj_fill_kernel");
-    BM_CUDA(ctx, cudaMemsetAsync(d_feat, 0, sizeof(int4) * ((size_t)n + 1), ctx->stream));
-    const size_t smem = sizeof(uint32_t) * (((size_t)n + 32) / 32);
-    if (smem > 48 * 1024)
-        BM_CUDA(ctx, cudaFuncSetAttribute(reach2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    reach2_kernel<<<ctx->num_sms * 4, kReachThreads, smem, ctx->stream>>>(Adj{d_optr, d_oidx}, Adj{d_iptr, d_iidx}, n,
-                                                                         d_next, d_feat);
+    const size_t smem = groups * 16;
+    // rows ORed at once: the fewest of up to eight that leave the fewest threads of the last step idle
+    int copies = 1;
+    auto idle = [&](int c) { return (double)((groups * c + kReachThreads - 1) / kReachThreads * kReachThreads) / (groups * c); };
+    for (int c = 2; c <= 8; c++)
+        if (idle(c) < idle(copies)) copies = c;
+    auto adj = [](const Fill& f) { return Adj{f.ptr, f.idx, f.cnt, f.row, reinterpret_cast<const uint4*>(f.rows)}; };
+    reach2_kernel<<<ctx->num_sms * 8, kReachThreads, smem, ctx->stream>>>(adj(w.d[0]), adj(w.d[1]), n, copies, w.misc,
+                                                                            feat);
     BM_LAUNCH_CHECK(ctx, "reach2_kernel");
-    feat.resize((size_t)n + 1);
-    BM_CUDA(ctx, cudaMemcpyAsync(feat.data(), d_feat, sizeof(int4) * ((size_t)n + 1), cudaMemcpyDeviceToHost,
-                                 ctx->stream));
     return BM_OK;
 }
 
@@ -343,13 +560,45 @@ extern "C" bm_status bm_greedy_match_dev(bm_ctx* ctx, int32_t n, int64_t mA, con
         (mB > 0 && (!srcB || !dstB)))
         return bm_fail(ctx, BM_INVALID_ARG, "bad edge arrays");
     BM_CUDA(ctx, cudaSetDevice(ctx->device));
-    DevBuf mem;
-    std::vector<int4> fa, fb;
+    const int64_t m = std::max(mA, mB);
+    int32_t heavy = std::max(64, n / 64);
+    Arena mem;
+    Work w;
+    for (;;) {
+        lay_out(mem, w, n, m, heavy);
+        if (bm_cuda_malloc((void**)&mem.mem, mem.used) == cudaSuccess) break;
+        cudaGetLastError();
+        mem.mem = nullptr;
+        if (heavy == INT32_MAX) return bm_fail(ctx, BM_OOM, "greedy matching: device allocation failed");
+        heavy = INT32_MAX;  // without the bit rows
+    }
+    lay_out(mem, w, n, m, heavy);
     bm_status s;
-    bool badA = false, badB = false;
-    if ((s = graph_features(ctx, mem, n, mA, srcA, dstA, fa, &badA)) != BM_OK) return s;
-    if (!badA && (s = graph_features(ctx, mem, n, mB, srcB, dstB, fb, &badB)) != BM_OK) return s;
-    if (badA || badB) {
+    BM_CUDA(ctx, cudaMemsetAsync(w.misc, 0, 4 * sizeof(int), ctx->stream));
+    BM_CUDA(ctx, cudaMemsetAsync(w.rank, 0, sizeof(int32_t) * 2 * ((size_t)n + 1), ctx->stream));
+    BM_CUDA(ctx, cudaMemsetAsync(w.pi, 0, sizeof(int32_t) * ((size_t)n + 1), ctx->stream));
+    if ((s = graph_features(ctx, w, n, mA, heavy, srcA, dstA, w.feat)) != BM_OK) return s;
+    if ((s = graph_features(ctx, w, n, mB, heavy, srcB, dstB, w.feat + (n + 1))) != BM_OK) return s;
+    const unsigned nb = (unsigned)((n + 255) / 256);
+    rank_kernel<<<dim3(nb, std::min(nb, 16u), 2), 256, 0, ctx->stream>>>(w.feat, n, w.rank);
+    BM_LAUNCH_CHECK(ctx, "rank_kernel");
+    sorted_kernel<<<nb, 256, 0, ctx->stream>>>(w.feat, w.rank, n, w.fa, w.ida, w.idb, w.cf, w.cpos, w.misc + 2);
+    BM_LAUNCH_CHECK(ctx, "sorted_kernel");
+    const size_t smem = sizeof(int32_t) * kRound * kList + ((size_t)n / 16 + 1) * 16;
+    BM_CUDA(ctx, cudaFuncSetAttribute(commit_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int32_t head = 0; head < n; head += kRound) {
+        const int32_t count = std::min(kRound, n - head);
+        shortlist_kernel<<<(count + kListThreads / 32 - 1) / (kListThreads / 32), kListThreads, 0, ctx->stream>>>(
+            w.fa, head, count, w.cf, w.cpos, w.misc + 2, w.list);
+        BM_LAUNCH_CHECK(ctx, "shortlist_kernel");
+        commit_kernel<<<1, kGreedyThreads, smem, ctx->stream>>>(w.fa, w.ida, w.idb, n, head, head + count, w.list, w.cf,
+                                                                w.cpos, w.misc + 2, w.pi);
+        BM_LAUNCH_CHECK(ctx, "commit_kernel");
+    }
+    int bad = 0;
+    BM_CUDA(ctx, cudaMemcpyAsync(&bad, w.misc + 1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (bad) {
         const int32_t* ends[4] = {srcA, dstA, srcB, dstB};
         const int64_t ms[4] = {mA, mA, mB, mB};
         for (int q = 0; q < 4; q++)
@@ -357,38 +606,7 @@ extern "C" bm_status bm_greedy_match_dev(bm_ctx* ctx, int32_t n, int64_t mA, con
                 if (ends[q][e] < 1 || ends[q][e] > n)
                     return bm_fail(ctx, BM_INVALID_ARG, "edge endpoint %d outside 1..%d", ends[q][e], n);
     }
-    BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    // both graphs' vertices by descending feature sum, ties by id
-    auto order = [&](const std::vector<int4>& f, std::vector<int32_t>& ids, std::vector<int4>& sorted) {
-        ids.resize((size_t)n);
-        std::iota(ids.begin(), ids.end(), 1);
-        auto total = [&](int32_t v) {
-            const int4& x = f[(size_t)v];
-            return (long long)x.x + x.y + x.z + x.w;
-        };
-        std::stable_sort(ids.begin(), ids.end(), [&](int32_t p, int32_t q) { return total(p) > total(q); });
-        sorted.resize((size_t)n);
-        for (int32_t i = 0; i < n; i++) sorted[(size_t)i] = f[(size_t)ids[(size_t)i]];
-    };
-    std::vector<int32_t> ida, idb;
-    std::vector<int4> sfa, sfb;
-    order(fa, ida, sfa);
-    order(fb, idb, sfb);
-    int4 *d_fa, *d_fb, *d_cf;
-    int32_t *d_ida, *d_idb, *d_pi, *d_cpos;
-    if (!mem.get(&d_fa, (size_t)n) || !mem.get(&d_fb, (size_t)n) || !mem.get(&d_ida, (size_t)n) ||
-        !mem.get(&d_idb, (size_t)n) || !mem.get(&d_pi, (size_t)n + 1) || !mem.get(&d_cf, (size_t)n) ||
-        !mem.get(&d_cpos, (size_t)n))
-        return bm_fail(ctx, BM_OOM, "greedy matching: device allocation failed");
-    BM_CUDA(ctx, cudaMemcpyAsync(d_fa, sfa.data(), sizeof(int4) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_fb, sfb.data(), sizeof(int4) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_ida, ida.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemcpyAsync(d_idb, idb.data(), sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, ctx->stream));
-    BM_CUDA(ctx, cudaMemsetAsync(d_pi, 0, sizeof(int32_t) * ((size_t)n + 1), ctx->stream));
-    const size_t smem = sizeof(uint32_t) * (((size_t)n + 31) / 32);
-    greedy_kernel<<<1, kGreedyThreads, smem, ctx->stream>>>(d_fa, d_ida, d_fb, d_idb, n, d_cf, d_cpos, d_pi);
-    BM_LAUNCH_CHECK(ctx, "greedy_kernel");
-    BM_CUDA(ctx, cudaMemcpyAsync(pi, d_pi, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, ctx->stream));
+    BM_CUDA(ctx, cudaMemcpyAsync(pi, w.pi, sizeof(int32_t) * ((size_t)n + 1), cudaMemcpyDeviceToHost, ctx->stream));
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return BM_OK;
 }
