@@ -90,15 +90,54 @@ extern "C" bm_status bm_device_memory(bm_ctx* ctx, uint64_t* free_bytes, uint64_
 // --------------------------------------------------------------- lifecycle
 
 static void free_graph(DevGraph& g) {
-    bm_cuda_free(g.out_ptr); bm_cuda_free(g.in_ptr);
-    bm_cuda_free(g.out_ent); bm_cuda_free(g.in_ent);
-    bm_cuda_free(g.self_w);
-    bm_cuda_free(g.out_twin); bm_cuda_free(g.in_twin);
-    bm_cuda_free(g.out_ent0); bm_cuda_free(g.in_ent0);
-    bm_cuda_free(g.out_twin0); bm_cuda_free(g.in_twin0);
-    bm_cuda_free(g.out_pos); bm_cuda_free(g.in_pos);
-    bm_cuda_free(g.hash);
+    bm_cuda_free(g.mem);
     g = DevGraph();
+}
+
+// A replaced graph's block of up to this size is kept for the next graph: a
+// block of a few MB costs as much to get and give back (0.6 ms) as laying out
+// 40,000 edges in it (0.45 ms).
+constexpr size_t kSpareGraph = (size_t)32 << 20;
+
+bm_status bm_graph_alloc(bm_ctx* ctx, DevGraph& G, bool side_b, int32_t n, size_t mo, size_t mi, size_t hash) {
+    char* base = nullptr;
+    size_t used = 0;
+    auto take = [&](auto** p, size_t count) {
+        using T = std::remove_reference_t<decltype(**p)>;
+        if (base) *p = reinterpret_cast<T*>(base + used);
+        used += (sizeof(T) * std::max<size_t>(count, 1) + 255) & ~(size_t)255;
+    };
+    auto lay_out = [&]() {
+        used = 0;
+        take(&G.out_ptr, (size_t)n + 2);
+        take(&G.in_ptr, (size_t)n + 2);
+        take(&G.self_w, (size_t)n + 1);
+        take(&G.out_ent, mo);
+        take(&G.in_ent, mi);
+        if (!side_b) return;
+        take(&G.out_ent0, mo);
+        take(&G.in_ent0, mi);
+        take(&G.out_twin, mo);
+        take(&G.in_twin, mi);
+        take(&G.out_twin0, mo);
+        take(&G.in_twin0, mi);
+        take(&G.out_pos, mo);
+        take(&G.in_pos, mi);
+        take(&G.hash, hash);
+    };
+    lay_out();
+    if (ctx->spare.mem && used <= ctx->spare.mem_bytes && ctx->spare.mem_bytes <= 4 * used) {
+        base = (char*)ctx->spare.mem;
+        used = ctx->spare.mem_bytes;
+        ctx->spare = DevGraph();
+    } else {
+        free_graph(ctx->spare);
+        BM_CUDA(ctx, bm_cuda_malloc(&base, used));
+    }
+    G.mem = base;
+    G.mem_bytes = used;
+    lay_out();
+    return BM_OK;
 }
 
 extern "C" bm_status bm_ctx_create(int device, bm_ctx** out) {
@@ -150,6 +189,7 @@ extern "C" void bm_ctx_destroy(bm_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     free_graph(ctx->g[0]);
     free_graph(ctx->g[1]);
+    free_graph(ctx->spare);
     bm_cuda_free(ctx->pi); bm_cuda_free(ctx->pinv); bm_cuda_free(ctx->ov); bm_cuda_free(ctx->ximg);
     bm_cuda_free(ctx->d_score);
     bm_cuda_free(ctx->stage);
@@ -220,11 +260,9 @@ bm_status bm_require_mapped(bm_ctx* ctx) {
 
 // ------------------------------------------------------------ graph upload
 
-template <typename T>
-static bm_status upload(bm_ctx* ctx, T** d, const T* h, size_t count) {
-    size_t bytes = sizeof(T) * (count > 0 ? count : 1);
-    BM_CUDA(ctx, bm_cuda_malloc((void**)d, bytes));
-    if (count > 0) BM_CUDA(ctx, cudaMemcpy(*d, h, sizeof(T) * count, cudaMemcpyHostToDevice));
+template <typename T, typename H>
+static bm_status upload(bm_ctx* ctx, T* d, const H& h) {
+    if (!h.empty()) BM_CUDA(ctx, cudaMemcpy(d, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice));
     return BM_OK;
 }
 
@@ -240,10 +278,24 @@ static bm_status upload(bm_ctx* ctx, T** d, const T* h, size_t count) {
 // two dozen launches and allocations cost the same for any list.
 constexpr int64_t kDeviceBuildMin = 8192;
 
-// The new graph of a side takes the place of the old one, whose mapping goes.
-static void adopt_graph(bm_ctx* ctx, int side, const DevGraph& built) {
+// What a side's old graph leaves behind when it is replaced: the mapping, and
+// the captured row launches, whose arguments name its arrays (a later graph may
+// start in the same block).
+static void drop_state(bm_ctx* ctx) {
     ctx->mapped = false;
-    free_graph(ctx->g[side]);
+    if (ctx->row_graph.exec) cudaGraphExecDestroy(ctx->row_graph.exec);
+    ctx->row_graph.exec = nullptr;
+}
+
+// The new graph of a side takes the place of the old one.
+static void adopt_graph(bm_ctx* ctx, int side, const DevGraph& built) {
+    drop_state(ctx);
+    if (ctx->g[side].mem && ctx->g[side].mem_bytes <= kSpareGraph) {
+        free_graph(ctx->spare);
+        ctx->spare = ctx->g[side];
+    } else {
+        free_graph(ctx->g[side]);
+    }
     ctx->g[side] = built;
     ctx->g[side].loaded = true;
     ctx->n = built.n;
@@ -280,39 +332,37 @@ extern "C" bm_status bm_set_graph(bm_ctx* ctx, int side, int32_t n, int64_t m, c
     BM_CUDA(ctx, cudaSetDevice(ctx->device));
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 
-    // Replacing a graph drops the mapping state.
-    ctx->mapped = false;
+    drop_state(ctx);
     free_graph(ctx->g[side]);
     DevGraph& G = ctx->g[side];
     G.n = n;
     G.m_out = H.m_out();
     G.m_in = H.m_in();
     G.m_real = H.m_real;
-    BM_TRY(upload(ctx, &G.out_ptr, H.optr.data(), H.optr.size()));
-    BM_TRY(upload(ctx, &G.in_ptr, H.iptr.data(), H.iptr.size()));
+    BM_TRY(bm_graph_alloc(ctx, G, side == BM_SIDE_B, n, H.oent.size(), H.ient.size(), H.htab.size()));
+    BM_TRY(upload(ctx, G.out_ptr, H.optr));
+    BM_TRY(upload(ctx, G.in_ptr, H.iptr));
     if (side == BM_SIDE_A) {
         // A's device lists in bank-spread order (the row kernel's scatter);
         // the host copy below keeps them sorted by neighbour id
-        std::vector<uint32_t> oe = H.oent, ie = H.ient;
+        std::vector<uint32_t> oe(H.oent.begin(), H.oent.end()), ie(H.ient.begin(), H.ient.end());
         bm_bank_spread_lists(H.optr, oe);
         bm_bank_spread_lists(H.iptr, ie);
-        BM_TRY(upload(ctx, &G.out_ent, oe.data(), oe.size()));
-        BM_TRY(upload(ctx, &G.in_ent, ie.data(), ie.size()));
+        BM_TRY(upload(ctx, G.out_ent, oe));
+        BM_TRY(upload(ctx, G.in_ent, ie));
     } else {
-        BM_TRY(upload(ctx, &G.out_ent, H.oent.data(), H.oent.size()));
-        BM_TRY(upload(ctx, &G.in_ent, H.ient.data(), H.ient.size()));
+        BM_TRY(upload(ctx, G.out_ent, H.oent));
+        BM_TRY(upload(ctx, G.in_ent, H.ient));
     }
-    BM_TRY(upload(ctx, &G.self_w, H.self.data(), H.self.size()));
-    if (side == BM_SIDE_B) {
-        BM_TRY(upload(ctx, &G.out_twin, H.otw.data(), H.otw.size()));
-        BM_TRY(upload(ctx, &G.in_twin, H.itw.data(), H.itw.size()));
-        BM_TRY(upload(ctx, &G.out_twin0, H.otw.data(), H.otw.size()));
-        BM_TRY(upload(ctx, &G.in_twin0, H.itw.data(), H.itw.size()));
-        BM_TRY(upload(ctx, &G.out_pos, H.otw.data(), H.otw.size()));  // sized here, written with the mapping
-        BM_TRY(upload(ctx, &G.in_pos, H.itw.data(), H.itw.size()));
-        BM_TRY(upload(ctx, &G.out_ent0, H.oent.data(), H.oent.size()));
-        BM_TRY(upload(ctx, &G.in_ent0, H.ient.data(), H.ient.size()));
-        BM_TRY(upload(ctx, &G.hash, H.htab.data(), H.htab.size()));
+    BM_TRY(upload(ctx, G.self_w, H.self));
+    if (side == BM_SIDE_B) {  // (positions are written with the mapping)
+        BM_TRY(upload(ctx, G.out_twin, H.otw));
+        BM_TRY(upload(ctx, G.in_twin, H.itw));
+        BM_TRY(upload(ctx, G.out_twin0, H.otw));
+        BM_TRY(upload(ctx, G.in_twin0, H.itw));
+        BM_TRY(upload(ctx, G.out_ent0, H.oent));
+        BM_TRY(upload(ctx, G.in_ent0, H.ient));
+        BM_TRY(upload(ctx, G.hash, H.htab));
         G.hash_log2 = H.hlog2;
     } else {
         ctx->hA_optr = H.optr;

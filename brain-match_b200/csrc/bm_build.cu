@@ -323,12 +323,6 @@ struct Arena {
     }
 };
 
-template <typename T>
-bm_status dev_new(bm_ctx* ctx, T** p, size_t count) {
-    BM_CUDA(ctx, bm_cuda_malloc(p, sizeof(T) * std::max<size_t>(count, 1)));
-    return BM_OK;
-}
-
 #define BUILD_TRY(x)                \
     do {                            \
         bm_status _s = (x);         \
@@ -422,9 +416,10 @@ bm_status bm_build_graph_dev(bm_ctx* ctx, bool side_b, int32_t n, int64_t m, con
     BUILD_TRY(sort_by(ctx, p1, p0, out_order, d_src, m, bits, hist, total));
     BUILD_TRY(sort_by(ctx, nullptr, p0, p1, d_src, m, bits, hist, total));
     BUILD_TRY(sort_by(ctx, p1, p0, in_order, d_dst, m, bits, hist, total));
-    BUILD_TRY(dev_new(ctx, &G.self_w, (size_t)n + 1));
-    BUILD_TRY(dev_new(ctx, &G.out_ptr, V));
-    BUILD_TRY(dev_new(ctx, &G.in_ptr, V));
+    int64_t cap = 0;
+    if (side_b)
+        for (cap = 1024, G.hash_log2 = 10; cap < 2 * (m + 1); cap <<= 1) G.hash_log2++;
+    BUILD_TRY(bm_graph_alloc(ctx, G, side_b, n, lists, lists, (size_t)cap));
     BM_CUDA(ctx, cudaMemsetAsync(G.self_w, 0, 4 * ((size_t)n + 1), sm));
     BM_CUDA(ctx, cudaMemsetAsync(ocnt, 0, 4 * V, sm));
     BM_CUDA(ctx, cudaMemsetAsync(icnt, 0, 4 * V, sm));
@@ -455,23 +450,9 @@ bm_status bm_build_graph_dev(bm_ctx* ctx, bool side_b, int32_t n, int64_t m, con
     G.max_deg = h.max_deg;
     G.max_wdeg = h.max_wdeg;
     G.has_self = h.has_self;
-    BUILD_TRY(dev_new(ctx, &G.out_ent, mo));
-    BUILD_TRY(dev_new(ctx, &G.in_ent, mi));
     uint32_t *oent, *ient;  // id-sorted
     int32_t* tmp = nullptr;
     if (side_b) {
-        BUILD_TRY(dev_new(ctx, &G.out_ent0, mo));
-        BUILD_TRY(dev_new(ctx, &G.in_ent0, mi));
-        BUILD_TRY(dev_new(ctx, &G.out_twin, mo));
-        BUILD_TRY(dev_new(ctx, &G.in_twin, mi));
-        BUILD_TRY(dev_new(ctx, &G.out_twin0, mo));
-        BUILD_TRY(dev_new(ctx, &G.in_twin0, mi));
-        BUILD_TRY(dev_new(ctx, &G.out_pos, mo));
-        BUILD_TRY(dev_new(ctx, &G.in_pos, mi));
-        int64_t cap = 1024;
-        G.hash_log2 = 10;
-        while (cap < 2 * (m + 1)) { cap <<= 1; G.hash_log2++; }
-        BUILD_TRY(dev_new(ctx, &G.hash, (size_t)cap));
         BM_CUDA(ctx, cudaMemsetAsync(G.hash, 0xFF, 8 * (size_t)cap, sm));
         BM_CUDA(ctx, cudaMemsetAsync(G.out_twin0, 0xFF, 4 * mo, sm));
         BM_CUDA(ctx, cudaMemsetAsync(G.in_twin0, 0xFF, 4 * mi, sm));

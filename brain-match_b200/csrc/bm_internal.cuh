@@ -36,6 +36,8 @@
 #include "bm_csr.hpp"
 
 struct DevGraph {
+    void* mem = nullptr;  // the one allocation that holds the arrays below
+    size_t mem_bytes = 0;
     int32_t n = 0;
     int64_t m_out = 0;   // out-list slots, including the null entries padding each list to 4
     int64_t m_in = 0;    // in-list slots
@@ -105,6 +107,7 @@ struct bm_ctx {
     int num_sms = 0;
     size_t smem_optin = 0;
     DevGraph g[2];
+    DevGraph spare;                 // the block of the graph replaced last, up to kSpareGraph bytes (bm_api.cu)
     int32_t n = 0;
     int32_t nvec = 0;               // n+1 rounded up to a multiple of 4 (vectorised per-vertex arrays)
     // mapping state (device)
@@ -329,6 +332,12 @@ __device__ __forceinline__ int32_t imin(int32_t a, int32_t b) { return a < b ? a
 __device__ __forceinline__ int4 bm_image_bounds(const int32_t* Bin_ptr, const int32_t* Bout_ptr, int32_t g) {
     return make_int4(Bin_ptr[g], Bin_ptr[g + 1], Bout_ptr[g], Bout_ptr[g + 1]);
 }
+
+// Device arrays of a graph with at most mo out-list and mi in-list slots (and
+// `hash` hash slots, side B), as one allocation.  With one for each array (0.33
+// ms to get, 0.3 ms to give back) they were 7 of the 12 ms that loading
+// 3,000,000 edges took.
+bm_status bm_graph_alloc(bm_ctx* ctx, DevGraph& G, bool side_b, int32_t n, size_t mo, size_t mi, size_t hash);
 
 // Kernel launchers implemented across the .cu files.
 bm_status bm_launch_score(bm_ctx* ctx, int64_t* score_out);

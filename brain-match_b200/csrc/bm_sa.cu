@@ -742,16 +742,15 @@ extern "C" bm_status bm_sa_run(bm_batch* b, int32_t nchains, const int32_t* chai
     }
     // per-chain state: mapping (input/output) and the per-vertex overlap (scratch)
     const int64_t tot = off[(size_t)nchains];
-    int32_t* d_pi = nullptr;
-    int32_t* d_ov = nullptr;
-    ChainDev* d_ch = nullptr;
-    BM_CUDA(ctx, bm_cuda_malloc(&d_pi, sizeof(int32_t) * (size_t)tot));
-    BM_CUDA(ctx, bm_cuda_malloc(&d_ov, sizeof(int32_t) * (size_t)tot));
-    BM_CUDA(ctx, bm_cuda_malloc(&d_ch, sizeof(ChainDev) * (size_t)nchains));
+    const size_t vec = (sizeof(int32_t) * (size_t)tot + 255) & ~(size_t)255;
     struct Guard {
-        void* p[3];
-        ~Guard() { for (void* x : p) bm_cuda_free(x); }
-    } guard{{d_pi, d_ov, d_ch}};
+        char* p = nullptr;
+        ~Guard() { bm_cuda_free(p); }
+    } mem;
+    BM_CUDA(ctx, bm_cuda_malloc(&mem.p, 2 * vec + sizeof(ChainDev) * (size_t)nchains));
+    int32_t* d_pi = reinterpret_cast<int32_t*>(mem.p);
+    int32_t* d_ov = reinterpret_cast<int32_t*>(mem.p + vec);
+    ChainDev* d_ch = reinterpret_cast<ChainDev*>(mem.p + 2 * vec);
     BM_CUDA(ctx, cudaMemcpyAsync(d_pi, init_pi, sizeof(int32_t) * (size_t)tot, cudaMemcpyHostToDevice, ctx->stream));
     BM_CUDA(ctx, cudaMemsetAsync(d_ov, 0, sizeof(int32_t) * (size_t)tot, ctx->stream));
     std::vector<ChainDev> hc((size_t)nchains);
