@@ -18,9 +18,9 @@
 // step counter moves past the accepted proposal, or by K when none is
 // accepted).  K starts at the tuned value and then follows the chain's
 // acceptances (up to 64), so long runs of rejections are evaluated 64 at a
-// time; the chain's mapping lives in shared memory when it fits.  A launch advances every chain by at most `chunk` proposals;
-// the launch is captured once in a CUDA graph and replayed until all chains
-// finish.
+// time; the chain's mapping lives in shared memory when it fits.  A launch
+// advances every chain by at most `chunk` proposals; the launch is captured
+// once in a CUDA graph and replayed until all chains finish.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -82,6 +82,7 @@ struct SaArgs {
 
 constexpr int kSaThreads = 512;     // threads per CTA of the allocation-free entry point (bm_sa_run tunes 256 or 512)
 constexpr int kSaMaxK = 64;         // proposals per iteration, adaptive up to this
+constexpr float kSaFixed = 15.f;    // twice an iteration's fixed part, in evaluations of a proposal (the rule of K)
 constexpr int kSaMaxInitialK = 16;  // largest settable starting K
 constexpr int kSaItem = 128;        // list entries per work item (four per lane)
 constexpr int kSaLongItem = 32;     // entries of an item whose row is longer than kSaRowCap: one hash lookup a lane takes as
@@ -170,17 +171,22 @@ __device__ void chain_apply_block(const PairDev& P, int32_t* pi, int32_t* gpi, i
 // than the buffer use the hash; a slot that two entries of the row share is
 // marked and searched.)  64 chains of 100,000 steps on four pairs of 2,709 to
 // 8,192 vertices: 107 ms with the searches and the staged swap apply, 88 ms
-// with the index, 84 ms with small items for the lists that use the hash; what
+// with the index, 83 ms with small items for the lists that use the hash; what
 // bounds an iteration now is the latency of its 16 warps an SM.  For an entry
 // of u whose other end is v, the direct-edge repair
 // min(w, B(pi u, pi v)) + min(w, B(pi v, pi u)) is added; the item sums meet in
 // a per-proposal shared counter, then
 //   delta = sum - S(u) - S(v) + self-loop terms.
 // The first accepted proposal in step order is applied and the rest are
-// discarded, so the chain is the one-at-a-time chain for every K.  K adapts
-// to the acceptance rate: it doubles (up to kSaMaxK) after an iteration with
-// no acceptance and drops to max(a.K, 2 (j + 1)) after the j-th proposal is
-// accepted; a function of the chain's own history, so replays are exact.
+// discarded, so the chain is the one-at-a-time chain for every K.  K follows
+// the mean number m of steps from one acceptance to the next (over about the
+// last eight, or since the last if that is longer): an iteration costs a fixed
+// part, as much as kSaFixed / 2 evaluations, and K evaluations, of which those
+// past the accepted one are lost, and sqrt(kSaFixed m) is near the K of least
+// cost.  Doubling K after an iteration without an acceptance, and twice the
+// accepted position after one, evaluated half the proposals in vain: 83.4 ms for
+// the run above, 79.0 so (kSaFixed 7: 79.9, 30: 81.8).  A function of the
+// chain's own history, so replays are exact.
 template <int CL, int THREADS>
 __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
     extern __shared__ __align__(16) uint32_t s_dyn[];
@@ -224,6 +230,7 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
     const uint64_t end = min(a.steps, step + a.chunk);
     long long score = ch.score, accepts = ch.accepts;
     int K = min(max(a.K, 1), kSaMaxK);
+    float mean = (float)(K * K) / kSaFixed, gap = 0;  // steps from one acceptance to the next; since the last one
     if (tid == 0) s_first = kSaMaxK;
     __syncthreads();
     while (step < end) {
@@ -467,15 +474,18 @@ __device__ __forceinline__ void sa_chain_body(const SaArgs& a) {
             score += s_d[first];
             accepts++;
             step += (uint64_t)first + 1;
-            K = min(kSaMaxK, max(a.K, 2 * (first + 1)));
+            mean += (gap + (float)(first + 1) - mean) * 0.125f;
+            gap = 0;
             chain_apply_block<CL>(P, pi, gpi, ov, pr.u, pr.v, crank);  // ends with a (cluster) barrier
             if (tid == 0) s_first = kSaMaxK;
         } else {
             step = min(end, step + (uint64_t)K);
-            K = min(kSaMaxK, 2 * K);
+            gap += (float)K;
+            mean = fmaxf(mean, gap);
             // the other CTA's reads of these sums end before they are reset
             if constexpr (CL > 1) cg::this_cluster().sync();
         }
+        K = min(kSaMaxK, max(a.K, __float2int_rn(sqrtf(kSaFixed * mean))));
         __syncthreads();
     }
     if (threadIdx.x == 0 && crank == 0) {

@@ -137,7 +137,8 @@ typedef struct bm_row_result {
  * no split plan) the call replays a CUDA graph whose kernels write the
  * results into pinned memory and returns as soon as every row's result has
  * arrived; the graph's last steps finish in the context's stream order
- * before any later work of the context. */
+ * before any later work of the context.  Other calls of up to 4,096 rows
+ * launch plainly and return in the same way. */
 bm_status bm_rows_best(bm_ctx* ctx, const int32_t* rows, const int32_t* col_lo,
                        int32_t nrows, bm_row_result* out);
 bm_status bm_rows_best_dev(bm_ctx* ctx, const int32_t* d_rows, const int32_t* d_col_lo,
@@ -285,8 +286,7 @@ typedef struct bm_sa_params {
                           * (with the CTAs per chain: 1, or a pair of CTAs when the chains fill at most
                           * half the SMs; the tuner times a prefix of the run for each choice and caches
                           * the best per device, sizes and chain count).  Each chain then adapts it (up
-                          * to 64) to its own acceptances: doubled after an iteration with none,
-                          * 2 (j + 1) after the j-th is accepted. */
+                          * to 64) to the mean distance of its own acceptances. */
     int64_t chunk;       /* proposals per chain per kernel launch (0 = 65536) */
     int32_t threads_per_cta; /* 256 or 512 with a set candidates value; 0 = 512 there, and with
                               * candidates = 0 the tuner chooses it as well (256 or 512) */
