@@ -16,8 +16,8 @@
 // kernel in its one-sided mode (the first two 2-hop terms only), read at the
 // members' columns; the assignment is solved by the auction algorithm
 // (Bertsekas) with epsilon scaling on benefits multiplied by k + 1, which makes
-// the final epsilon = 1 phase exactly optimal for integer benefits, in one CTA
-// with prices, bids and owners in shared memory; apply_perm_kernel then moves
+// the final epsilon = 1 phase exactly optimal for integer benefits, with prices,
+// bids and owners in one CTA's shared memory; apply_perm_kernel then moves
 // every changed member at once (S updates of its A entries, relabelled B
 // entries naming its new image, pi and pi^-1).
 #include <algorithm>
@@ -48,16 +48,16 @@ constexpr long long kAuctionLimit = 20000000000ll;
 // many bidders the CTAs of its cluster share their rows (each reads the prices
 // and places its bids through distributed shared memory), since one SM reads
 // the benefits at a small part of the L2's rate.  Every round all unassigned
-// persons bid at the same prices; of a random subset's assignment three rounds in four have a single
-// bidder (a chain of displaced persons), so a round's fixed cost is what bounds
-// it: the list of bidders is carried from round to round instead of being
+// persons bid at the same prices; of a random subset's assignment three rounds
+// in four have a single bidder (a chain of displaced persons), so a round's
+// fixed cost is what bounds it: the list of bidders is carried from round to round instead of being
 // searched for among all persons, the warps share the rows of few bidders
 // (all 32 one row when there is one), and only the objects that got a bid are
 // visited.  Values and prices are computed in 32 bits while they stay below
 // 2^30 (benefits times k + 1 and every bid, checked), else in 64: the same
-// integers, and the same assignment as one CTA's.  k = 1,542 of the full-scale pair: 33.5 ms with a warp a row and
-// the searches and one CTA throughout, 14.6 ms in one CTA as it is now, 13 ms
-// with the cluster.
+// integers, and the same assignment as one CTA's.  k = 1,542 of the full-scale
+// pair: 33.5 ms with a warp a row and the searches and one CTA throughout, 14.6
+// ms in one CTA as it is now, 13 ms with the cluster.
 struct AuctionSmem {
     unsigned long long* bid;  // per object: bid << kLapIdBits | reversed person, 0: none
     int32_t* owner;           // per object

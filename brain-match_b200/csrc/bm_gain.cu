@@ -18,8 +18,8 @@
 // the roles of rows and columns changed), consecutive threads on consecutive
 // columns: the late swaps of a search are its hubs', whose lists cover much of
 // a row, and updates in list order, a 32-byte sector each, took 431 us a batch
-// of swaps of the full-scale search against 166 with the lists.  Then the swap itself: columns a and b of T change places,
-// and rows of H by hrow.
+// of swaps of the full-scale search against 140 with the lists.  Then the swap
+// itself: columns a and b of T change places, and rows of H by hrow.
 //
 // A search that accepts thousands of swaps a pass is better off scattering
 // rows; one that accepts a few hundred and fewer is not (bm_gains_pay).
