@@ -533,7 +533,7 @@ static bm_status bm_table_topk_launch(bm_ctx* ctx, const int32_t* d_tab, int64_t
 }
 
 static bool small_table(const bm_ctx* ctx) {
-    double work = 9e4 * ctx->n;
+    double work = 6e4 * ctx->n;
     if (work >= 1.8e8) return false;
     for (int32_t w : ctx->h_rwork) work += w;
     return work < 1.8e8;
@@ -553,10 +553,10 @@ extern "C" bm_status bm_delta_table_dev(bm_ctx* ctx, int32_t* d_table, int64_t l
     // the reference-delta terms of self-loops are per row, and rows that do not
     // start on 16-byte boundaries have no vector access: those keep the row
     // kernel's own finish.  So do small tables, which do not repay the two more
-    // launches: those cost 30 us against 15 ns a row and 0.17 us a million 2-hop
+    // launches: those cost 30 us against 10 ns a row and 0.17 us a million 2-hop
     // entries saved (500 vertices, 24,000 edges: 49 us two-sided, 70 one-sided;
     // 1,000 and 60,000: 80 and 96; 1,000 and 125,000: 127 and 116; 2,000 and
-    // 40,000: 124 and 117).
+    // 40,000: 124 and 117; 2,348 and 63,396, with the top 2,132: 666 and 671).
     const bool refcpu = ctx->semantics == BM_SEMANTICS_REF_CPU && A.has_self;
     if (refcpu || (ld & 3) != 0 || ((uintptr_t)d_table & 15) != 0 || small_table(ctx))
         return bm_launch_rows_ex(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0);

@@ -10,7 +10,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("n,m", [(700, 1000), (700, 180_000), (1999, 4000), (2000, 4000), (2047, 6000), (2048, 6000),
-                                 (2049, 9000), (2113, 200_000)])
+                                 (2049, 9000), (2113, 200_000), (2999, 4000), (3000, 4000), (3007, 5000), (3008, 5000),
+                                 (3009, 5000)])
 def test_both_sides(n, m):
     rng = np.random.default_rng(n + m)
 
