@@ -177,7 +177,7 @@ struct GroupArgs {
     const int32_t* item0;    // u's first item (n + 1)
     const int32_t* item_u;   // u of an item
     const int32_t* nitems;
-    int32_t* next;           // claim counter
+    int32_t* next;           // claims of items past the blocks' first ones
     const int2* sorted;      // {v, index} by u
     int64_t* out;
 };
@@ -286,9 +286,10 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpThreads == 1024 ? 1 : 2) pair
     const GView& A = a.p.A;
     for (int32_t i = tid; i < a.nv / 2; i += kGrpThreads) reinterpret_cast<uint4*>(gsm)[i] = make_uint4(0, 0, 0, 0);
     const int32_t nitems = __ldg(a.nitems);
-    if (tid == 0) s_item = atomicAdd(a.next, 1);
     __syncthreads();
-    int32_t item = s_item;
+    // a block's first item is its own number, the later ones are claimed: s_item is
+    // written only at the head of an item and read between its barriers
+    int32_t item = (int32_t)blockIdx.x;
     while (item < nitems) {
         const int32_t u = __ldg(a.item_u + item);
         const int32_t p0 = __ldg(a.off + u) + (item - __ldg(a.item0 + u)) * kGrpPairs;
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(kGrpThreads, kGrpThreads == 1024 ? 1 : 2) pair
         const int4 xu = __ldg(a.ximg + u);
         const int32_t uo0 = __ldg(A.out_ptr + u), uo1 = __ldg(A.out_ptr + u + 1);
         const int32_t ui0 = __ldg(A.in_ptr + u), ui1 = __ldg(A.in_ptr + u + 1);
-        if (tid == 0) { s_item = atomicAdd(a.next, 1); s_claim = 0; }
+        if (tid == 0) { s_item = (int32_t)gridDim.x + atomicAdd(a.next, 1); s_claim = 0; }
         table_list<kGrpThreads>(T0, a.Aout, uo0, uo1, true);
         table_list<kGrpThreads>(T1, a.Ain, ui0, ui1, true);
         table_list<kGrpThreads>(T2, a.Bout, xu.z, xu.w, true);
