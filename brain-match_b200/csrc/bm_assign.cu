@@ -211,8 +211,9 @@ __device__ int auction_rounds(const int32_t* __restrict__ a, int32_t k, const Au
         while (nu > 0) {
             if (nu == 1) {
                 // a chain: the bidder takes its best object unopposed and whoever
-                // held that bids next
-                if (tid == 0 && clock64() - t0 > limit) *s_flag = 1;
+                // held that bids next.  The round ends with its flag and count being
+                // read and no barrier behind that, so both are written between the
+                // two barriers only, the clock's verdict too
                 const int32_t i = s.list[cur][0];
                 Top2<T> t = scan_row<kLapMaxK / kLapThreads>(a, price, k, scale, i, tid, kLapThreads);
                 warp_merge(t);
@@ -222,11 +223,11 @@ __device__ int auction_rounds(const int32_t* __restrict__ a, int32_t k, const Au
                     t = part[lane];
                     warp_merge(t);
                     if (lane == 0) {
-                        const int st = place_bid(s, price, t, 0, i, eps);
+                        const int st = clock64() - t0 > limit ? 1 : place_bid(s, price, t, 0, i, eps);
                         const int32_t j = t.j1;
                         if (st) {
                             *s_flag = st;
-                        } else if (*s_flag == 0) {
+                        } else {
                             price[j] = (T)(long long)(s.bid[j] >> kLapIdBits);
                             const int32_t old = s.owner[j];
                             s.owner[j] = i;
