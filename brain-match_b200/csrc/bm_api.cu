@@ -196,6 +196,7 @@ extern "C" void bm_ctx_destroy(bm_ctx* ctx) {
     bm_cuda_free(ctx->flush_buf);
     bm_cuda_free(ctx->tscr);
     bm_cuda_free(ctx->pscr);
+    for (void* p : ctx->pscr_old) bm_cuda_free(p);
     bm_cuda_free(ctx->rwork); bm_cuda_free(ctx->spart); bm_cuda_free(ctx->scnt); bm_cuda_free(ctx->rpart); bm_cuda_free(ctx->slots);
     if (ctx->hstage) bm_cuda_host_free(ctx->hstage);
     if (ctx->h_slots) bm_cuda_host_free(ctx->h_slots);
@@ -278,11 +279,13 @@ static bm_status upload(bm_ctx* ctx, T* d, const H& h) {
 // two dozen launches and allocations cost the same for any list.
 constexpr int64_t kDeviceBuildMin = 8192;
 
-// What a side's old graph leaves behind when it is replaced: the mapping, and
-// the captured row launches, whose arguments name its arrays (a later graph may
-// start in the same block).
+// What a side's old graph leaves behind when it is replaced: the mapping, the
+// captured row launches, whose arguments name its arrays (a later graph may
+// start in the same block), and outgrown scratch.  The stream is idle.
 static void drop_state(bm_ctx* ctx) {
     ctx->mapped = false;
+    for (void* p : ctx->pscr_old) bm_cuda_free(p);
+    ctx->pscr_old.clear();
     if (ctx->row_graph.exec) cudaGraphExecDestroy(ctx->row_graph.exec);
     ctx->row_graph.exec = nullptr;
 }

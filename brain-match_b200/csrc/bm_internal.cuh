@@ -132,6 +132,7 @@ struct bm_ctx {
     size_t tscr_bytes = 0;
     void* pscr = nullptr;           // scratch of grouped pair deltas (bm_pairs.cu), bounded
     size_t pscr_bytes = 0;
+    std::vector<void*> pscr_old;    // outgrown blocks of it, given back when the stream is idle
     int64_t launches = 0;
     int32_t row_ctas = 0;           // CTAs per row (cluster size); 0 = auto
     int32_t row_threads = 512;

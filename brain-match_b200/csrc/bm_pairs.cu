@@ -434,20 +434,25 @@ bool use_groups(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t run) {
     const double items = (double)std::min<int64_t>(ctx->n, (k + run - 1) / run);
     const double entries = 2.0 * (double)(ctx->g[0].m_out + ctx->g[0].m_in) / ctx->n;  // of an average pair
     if ((double)k * entries * 0.02 < 29.0 * items || k < 1024) return false;
-    const size_t need = GroupScratch(ctx->n, std::min(k, kGrpChunk)).total;
-    if (ctx->pscr_bytes >= need) return true;
-    // growing the scratch waits for the stream, which a capture does not allow
+    // the scratch is the context's: a capture's later replays would share it with
+    // whatever call comes then
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-    if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
-    bm_cuda_free(ctx->pscr);
-    ctx->pscr = nullptr;
-    ctx->pscr_bytes = 0;
-    if (bm_cuda_malloc(&ctx->pscr, need) != cudaSuccess) {
+    const size_t need = GroupScratch(ctx->n, std::min(k, kGrpChunk)).total;
+    if (ctx->pscr_bytes >= need) return true;
+    // The call does not wait for the device: an outgrown block, which launches
+    // in flight may use, is put by until the stream is next idle (bm_set_graph).
+    // Blocks double up to the largest, so those put by hold about as much
+    // together as the one in use at most.
+    const size_t most = GroupScratch(ctx->n, kGrpChunk).total, size = std::max(need, std::min(most, 2 * ctx->pscr_bytes));
+    void* block = nullptr;
+    if (bm_cuda_malloc(&block, size) != cudaSuccess) {
         cudaGetLastError();  // no room for the sort: one warp per pair needs none
         return false;
     }
-    ctx->pscr_bytes = need;
+    if (ctx->pscr) ctx->pscr_old.push_back(ctx->pscr);
+    ctx->pscr = block;
+    ctx->pscr_bytes = size;
     return true;
 }
 

@@ -112,7 +112,10 @@ bm_status bm_get_overlap(bm_ctx* ctx, int32_t* ov);
  * calculateSwapDeltasKernel(Quick) (src/graph-re-alignment-gpu.cu:46-248).
  * u == v gives 0. */
 bm_status bm_delta_pairs(bm_ctx* ctx, const int32_t* pairs, int64_t k, int64_t* deltas);
-/* Same, device pointers, asynchronous on the context stream. */
+/* Same, device pointers, asynchronous on the context stream.  Long lists are
+ * sorted in scratch that the context keeps (8 bytes a pair, at most 34 MB, and
+ * as much again in outgrown blocks until a graph is next set); a call that is
+ * being captured uses none. */
 bm_status bm_delta_pairs_dev(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_deltas);
 
 /* Exact deltas of whole rows: for each row u = rows[r], delta(u, v) for
