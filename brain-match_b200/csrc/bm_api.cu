@@ -681,6 +681,21 @@ extern "C" bm_status bm_get_row_tiers(bm_ctx* ctx, int32_t* heavy_rows) {
     return BM_OK;
 }
 
+extern "C" bm_status bm_set_path(bm_ctx* ctx, int32_t path, int32_t mode) {
+    if (!ctx) return BM_INVALID_ARG;
+    if (path < 0 || path >= BM_PATHS || mode < -1 || mode > 1)
+        return bm_fail(ctx, BM_INVALID_ARG, "path must be 0..%d and mode -1 (never), 0 (by the rule) or 1 (always)", BM_PATHS - 1);
+    ctx->path[path] = mode;
+    return BM_OK;
+}
+
+extern "C" bm_status bm_get_path(bm_ctx* ctx, int32_t path, int32_t* mode) {
+    if (!ctx || !mode) return BM_INVALID_ARG;
+    if (path < 0 || path >= BM_PATHS) return bm_fail(ctx, BM_INVALID_ARG, "path must be 0..%d", BM_PATHS - 1);
+    *mode = ctx->path[path];
+    return BM_OK;
+}
+
 extern "C" bm_status bm_get_row_tiling(bm_ctx* ctx, int32_t* ctas_per_row, int32_t* threads) {
     if (!ctx) return BM_INVALID_ARG;
     if (ctas_per_row) *ctas_per_row = ctx->row_ctas;

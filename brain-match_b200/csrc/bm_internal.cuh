@@ -139,6 +139,7 @@ struct bm_ctx {
     // split rows (bm_rows.cu): per-row work estimate, slot partial sums,
     // self-resetting arrival counters and slice reductions
     int32_t row_split = 0;          // 0 = automatic slots, -1 = off, k > 0 = k slots
+    int32_t path[BM_PATHS] = {0};   // bm_set_path
     int32_t semantics = 0;          // BM_SEMANTICS_EXACT or BM_SEMANTICS_REF_CPU (pairwise swap deltas)
     int32_t* rwork = nullptr;
     std::vector<int32_t> h_rwork;   // host copy (the split plan is made on the host)

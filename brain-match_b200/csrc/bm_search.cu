@@ -277,9 +277,15 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
         BmGains g;
         ~GainsGuard() { bm_gains_free(&g); }
     } gains;
-    const bool may_gain = bm_gains_possible(ctx);
+    const int32_t gain_mode = ctx->path[BM_PATH_GAIN_TABLES];
+    const bool may_gain = gain_mode >= 0 && bm_gains_possible(ctx);
     bool no_room = false;
     const auto t0 = clk::now();
+    if (may_gain && gain_mode > 0) {
+        bool ok = false;
+        if ((s = bm_gains_build(ctx, &gains.g, &ok)) != BM_OK) return s;
+        no_room = !ok;
+    }
     int32_t pos = prog->next_row_pos;
     if (pos < 0 || pos >= nr) pos = 0;
     bool pass_full = (pos == 0);

@@ -170,6 +170,8 @@ def cuda_lib() -> C.CDLL:
             "bm_set_row_tiling": (C.c_int, [vp, C.c_int32, C.c_int32]),
             "bm_set_row_split": (C.c_int, [vp, C.c_int32]),
             "bm_set_row_tiers": (C.c_int, [vp, C.c_int32]),
+            "bm_set_path": (C.c_int, [vp, C.c_int32, C.c_int32]),
+            "bm_get_path": (C.c_int, [vp, C.c_int32, C.POINTER(C.c_int32)]),
             "bm_get_row_tiers": (C.c_int, [vp, C.POINTER(C.c_int32)]),
             "bm_set_semantics": (C.c_int, [vp, C.c_int32]),
             "bm_get_semantics": (C.c_int, [vp, C.POINTER(C.c_int32)]),
@@ -724,6 +726,17 @@ class Engine:
     def row_tiers(self) -> int:
         v = C.c_int32()
         self._chk(self.L.bm_get_row_tiers(self.h, C.byref(v)), "bm_get_row_tiers")
+        return v.value
+
+    PATHS = {"gain_tables": 0}
+
+    def set_path(self, path: str, mode: int = 0) -> None:
+        """A path that a rule chooses: 0 by the rule, 1 wherever possible, -1 never."""
+        self._chk(self.L.bm_set_path(self.h, self.PATHS[path], mode), "bm_set_path")
+
+    def path(self, path: str) -> int:
+        v = C.c_int32()
+        self._chk(self.L.bm_get_path(self.h, self.PATHS[path], C.byref(v)), "bm_get_path")
         return v.value
 
     SEMANTICS = {"exact": 0, "ref-cpu": 1}

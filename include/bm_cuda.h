@@ -666,6 +666,17 @@ bm_status bm_get_row_split(bm_ctx* ctx, int32_t* slots);
  * split plan is active.  No reference counterpart. */
 bm_status bm_set_row_tiers(bm_ctx* ctx, int32_t heavy_rows);
 bm_status bm_get_row_tiers(bm_ctx* ctx, int32_t* heavy_rows);
+/* Paths that a rule on sizes chooses, each with the same results as what it
+ * stands in for: 0 = by the rule (default), 1 = wherever the path can be taken,
+ * -1 = never.  BM_PATH_GAIN_TABLES: bm_search_batched keeps the one-sided gains
+ * of all rows in two n x n tables and reads its batches from them (not with
+ * repeated A edges, nor with self-loops of A under BM_SEMANTICS_REF_CPU, nor
+ * beyond about 57,000 vertices or half of the free device memory).  A testing
+ * and diagnosis aid; no reference counterpart. */
+#define BM_PATH_GAIN_TABLES 0
+#define BM_PATHS 1
+bm_status bm_set_path(bm_ctx* ctx, int32_t path, int32_t mode);
+bm_status bm_get_path(bm_ctx* ctx, int32_t path, int32_t* mode);
 /* How many row clusters of the given shape can be resident at once on the
  * device for the current n (cudaOccupancyMaxActiveClusters). */
 bm_status bm_rows_max_active_clusters(bm_ctx* ctx, int32_t ctas_per_row, int32_t threads, int32_t* out);
