@@ -558,7 +558,8 @@ extern "C" bm_status bm_delta_table_dev(bm_ctx* ctx, int32_t* d_table, int64_t l
     // 1,000 and 60,000: 80 and 96; 1,000 and 125,000: 127 and 116; 2,000 and
     // 40,000: 124 and 117; 2,348 and 63,396, with the top 2,132: 666 and 671).
     const bool refcpu = ctx->semantics == BM_SEMANTICS_REF_CPU && A.has_self;
-    if (refcpu || (ld & 3) != 0 || ((uintptr_t)d_table & 15) != 0 || small_table(ctx))
+    const int32_t mode = ctx->path[BM_PATH_TABLE_GAINS];
+    if (refcpu || (ld & 3) != 0 || ((uintptr_t)d_table & 15) != 0 || mode < 0 || (mode == 0 && small_table(ctx)))
         return bm_launch_rows_ex(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0);
     if ((s = bm_launch_rows_gen(ctx, d_rows, nullptr, n, nullptr, nullptr, d_table, ld, 0, nullptr, 0, nullptr, nullptr,
                                 true)) != BM_OK)
