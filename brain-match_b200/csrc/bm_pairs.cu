@@ -429,11 +429,12 @@ struct GroupScratch {
 // its items, at most one per u, cost less than the pairs' entries.  Lists with
 // repeated neighbours have no dense table; the tables must fit in shared memory.
 bool use_groups(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t run) {
-    if (ctx->g[0].has_dup || ((uintptr_t)d_pairs & 7)) return false;
+    const int32_t mode = ctx->path[BM_PATH_PAIR_GROUPS];
+    if (mode < 0 || ctx->g[0].has_dup || ((uintptr_t)d_pairs & 7)) return false;
     if (group_smem(ctx->n) + 16384 > ctx->smem_optin) return false;
     const double items = (double)std::min<int64_t>(ctx->n, (k + run - 1) / run);
     const double entries = 2.0 * (double)(ctx->g[0].m_out + ctx->g[0].m_in) / ctx->n;  // of an average pair
-    if ((double)k * entries * 0.02 < 29.0 * items || k < 1024) return false;
+    if (mode == 0 && ((double)k * entries * 0.02 < 29.0 * items || k < 1024)) return false;
     // the scratch is the context's: a capture's later replays would share it with
     // whatever call comes then
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;

@@ -728,7 +728,7 @@ class Engine:
         self._chk(self.L.bm_get_row_tiers(self.h, C.byref(v)), "bm_get_row_tiers")
         return v.value
 
-    PATHS = {"gain_tables": 0, "table_gains": 1}
+    PATHS = {"gain_tables": 0, "table_gains": 1, "pair_groups": 2}
 
     def set_path(self, path: str, mode: int = 0) -> None:
         """A path that a rule chooses: 0 by the rule, 1 wherever possible, -1 never."""

@@ -674,11 +674,14 @@ bm_status bm_get_row_tiers(bm_ctx* ctx, int32_t* heavy_rows);
  * beyond about 57,000 vertices or half of the free device memory).
  * BM_PATH_TABLE_GAINS: bm_delta_table_dev scatters one-sided gains and adds the
  * table to its transpose (not with rows off 16-byte boundaries, nor with
- * self-loops of A under BM_SEMANTICS_REF_CPU).  A testing and diagnosis aid;
- * no reference counterpart. */
+ * self-loops of A under BM_SEMANTICS_REF_CPU).  BM_PATH_PAIR_GROUPS: pair deltas
+ * are sorted by their first vertex (not with repeated A edges, pairs off 8-byte
+ * boundaries, more than about 27,000 vertices, or while captured).  A testing
+ * and diagnosis aid; no reference counterpart. */
 #define BM_PATH_GAIN_TABLES 0
 #define BM_PATH_TABLE_GAINS 1
-#define BM_PATHS 2
+#define BM_PATH_PAIR_GROUPS 2
+#define BM_PATHS 3
 bm_status bm_set_path(bm_ctx* ctx, int32_t path, int32_t mode);
 bm_status bm_get_path(bm_ctx* ctx, int32_t path, int32_t* mode);
 /* How many row clusters of the given shape can be resident at once on the
