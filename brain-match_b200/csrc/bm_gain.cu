@@ -317,21 +317,25 @@ bool bm_gains_possible(bm_ctx* ctx) {
 }
 
 // In units of scattered 2-hop entries (1.9e12 a second on a B200): a pass over
-// all rows scatters W of them; reading the tables costs about 4 a table entry,
-// and an entry of a swap's product 4.  Products are taken as 64 times mean
-// lists' (late swaps are hubs').  Filling the tables costs about half a pass;
-// it has to come back within the next four passes, or those that are left
-// (`passes`, -1: no limit), and so has what does not depend on the sizes, the
-// allocation, its release and the launches, about half a millisecond (five
-// passes over 524 vertices: 1.47 ms with the tables, 0.90 ms without).
-bool bm_gains_pay(const bm_ctx* ctx, int64_t pass_accepts, int32_t passes) {
-    double W = 0;
+// the search's rows scatters theirs, `scatter` together; reading the tables
+// costs about 4 a table entry, and an entry of a swap's product 4.  Products are
+// taken as 64 times mean lists' (late swaps are hubs').  Filling the tables
+// costs about half a pass over all W entries of the graph, whatever rows the
+// search visits; it has to come back within the next four passes, or those that
+// are left (`passes`, -1: no limit), and so has what does not depend on the
+// sizes, the allocation, its release and the launches, about half a millisecond
+// (five passes over 524 vertices: 1.47 ms with the tables, 0.90 ms without).
+bool bm_gains_pay(const bm_ctx* ctx, const std::vector<int32_t>& order, int64_t pass_accepts, int32_t passes) {
+    if (ctx->h_rwork.size() != (size_t)ctx->n + 1) return false;
+    double W = 0, scatter = 0;
     for (int32_t w : ctx->h_rwork) W += w;
+    for (int32_t u : order) scatter += ctx->h_rwork[(size_t)u];
     const double n = ctx->n, d = (double)ctx->g[0].m_out / n, db = (double)ctx->g[1].m_out / n;
     const double update = 64.0 * d * db * 4.0;
     const double r = passes < 0 ? 4.0 : std::min(4, passes);
     const double fixed = 1e9;
-    return r * ((double)pass_accepts * update + 4.0 * n * n) + 0.45 * W + 4.0 * n * n + fixed < 0.9 * r * W;
+    return r * ((double)pass_accepts * update + 4.0 * n * (double)order.size()) + 0.45 * W + 4.0 * n * n + fixed <
+           0.9 * r * scatter;
 }
 
 // Fills the tables for the current mapping.  *ok is false, and nothing is

@@ -361,7 +361,7 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
                 } else if (max_sweeps >= 0 && prog->sweeps >= max_sweeps) {
                     done = true;
                 } else if (pass_full && may_gain && !no_room && !gains.g.held() &&
-                           bm_gains_pay(ctx, pass_accepts, max_sweeps < 0 ? -1 : max_sweeps - prog->sweeps)) {
+                           bm_gains_pay(ctx, order, pass_accepts, max_sweeps < 0 ? -1 : max_sweeps - prog->sweeps)) {
                     bool ok = false;
                     if ((s = bm_gains_build(ctx, &gains.g, &ok)) != BM_OK) return s;
                     no_room = !ok;
