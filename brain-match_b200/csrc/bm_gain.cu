@@ -325,14 +325,14 @@ bool bm_gains_possible(bm_ctx* ctx) {
 // are left (`passes`, -1: no limit), and so has what does not depend on the
 // sizes, the allocation, its release and the launches, about half a millisecond
 // (five passes over 524 vertices: 1.47 ms with the tables, 0.90 ms without).
-bool bm_gains_pay(const bm_ctx* ctx, const std::vector<int32_t>& order, int64_t pass_accepts, int32_t passes) {
+bool bm_gains_pay(const bm_ctx* ctx, const std::vector<int32_t>& order, int64_t pass_accepts, double passes) {
     if (ctx->h_rwork.size() != (size_t)ctx->n + 1) return false;
     double W = 0, scatter = 0;
     for (int32_t w : ctx->h_rwork) W += w;
     for (int32_t u : order) scatter += ctx->h_rwork[(size_t)u];
     const double n = ctx->n, d = (double)ctx->g[0].m_out / n, db = (double)ctx->g[1].m_out / n;
     const double update = 64.0 * d * db * 4.0;
-    const double r = passes < 0 ? 4.0 : std::min(4, passes);
+    const double r = passes < 0 ? 4.0 : std::min(4.0, passes);
     const double fixed = 1e9;
     return r * ((double)pass_accepts * update + 4.0 * n * (double)order.size()) + 0.45 * W + 4.0 * n * n + fixed <
            0.9 * r * scatter;

@@ -400,7 +400,7 @@ struct BmGains {
 };
 void bm_gains_free(BmGains* g);
 bool bm_gains_possible(bm_ctx* ctx);
-bool bm_gains_pay(const bm_ctx* ctx, const std::vector<int32_t>& order, int64_t pass_accepts, int32_t passes);
+bool bm_gains_pay(const bm_ctx* ctx, const std::vector<int32_t>& order, int64_t pass_accepts, double passes);
 bm_status bm_gains_build(bm_ctx* ctx, BmGains* g, bool* ok);
 bm_status bm_gains_rows_best(bm_ctx* ctx, const BmGains& g, const int32_t* d_rows, int32_t nrows, bm_row_result* d_res);
 bm_status bm_gains_apply(bm_ctx* ctx, const BmGains& g, const int32_t* d_pairs, int32_t k);

@@ -18,8 +18,9 @@
 // Independent swaps do not change each other's deltas, so the tracked score
 // stays exact.  Two things are done ahead of need there, without changing a
 // result.  Several batches are evaluated in one launch while batches accept
-// nothing (doubling, halved by an accept); they are consumed in order, and what
-// follows an accept is discarded and evaluated again.  And once a pass accepts
+// nothing (doubling, halved by an accept, no more than a time budget has room
+// for); they are consumed in order, and what follows an accept is discarded and
+// evaluated again.  And once a pass accepts
 // few swaps, the gains of all rows are kept in tables (bm_gain.cu), so that a
 // batch is read instead of scattered.  The full-scale search from the greedy
 // start (60 passes, the last 50 with 146 accepts and fewer) took 735-755 ms with
@@ -291,6 +292,8 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
     bool pass_full = (pos == 0);
     int64_t pass_accepts = 0, accepts0 = prog->accepts;
     int32_t ahead = 1;  // batches of a launch
+    double batch_s = 0;  // the longest batch so far, of those read from tables once there are some
+    double pass_t = 0;   // when the pass began
     prog->converged = 0;
     bm_status ret = BM_OK;
     auto stop = [&]() -> bool {
@@ -302,6 +305,9 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
     bool done = false;
     while (!done) {
         if (stop()) break;
+        const double launch_t = secs_since(t0);
+        if (time_budget_s > 0 && batch_s * ahead > time_budget_s - launch_t)
+            ahead = (int32_t)std::max(1.0, (time_budget_s - launch_t) / batch_s);
         const int32_t held = (int32_t)std::min<int64_t>((int64_t)R * ahead, nr - pos);  // rows of the launch
         for (int32_t i = 0; i < held; i++) b.h_rows[i] = order[(size_t)(pos + i)];
         if (gains.g.held()) {
@@ -312,6 +318,7 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
         } else if ((s = eval_rows(ctx, b, held, false)) != BM_OK) {
             return s;
         }
+        batch_s = std::max(batch_s, (secs_since(t0) - launch_t) * R / std::max(held, R));
         int32_t na = 0;
         for (int32_t r0 = 0; r0 < held && na == 0 && !done; r0 += R) {
             if (r0 > 0 && stop()) { done = true; break; }
@@ -360,12 +367,21 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
                     done = true;
                 } else if (max_sweeps >= 0 && prog->sweeps >= max_sweeps) {
                     done = true;
-                } else if (pass_full && may_gain && !no_room && !gains.g.held() &&
-                           bm_gains_pay(ctx, order, pass_accepts, max_sweeps < 0 ? -1 : max_sweeps - prog->sweeps)) {
-                    bool ok = false;
-                    if ((s = bm_gains_build(ctx, &gains.g, &ok)) != BM_OK) return s;
-                    no_room = !ok;
+                } else if (pass_full && may_gain && !no_room && !gains.g.held()) {
+                    // passes still to come, by the time that this one took where time is bounded
+                    double left = max_sweeps < 0 ? -1.0 : max_sweeps - prog->sweeps;
+                    if (time_budget_s > 0) {
+                        const double now = secs_since(t0), fit = std::max(0.0, time_budget_s - now) / (now - pass_t);
+                        left = left < 0 ? fit : std::min(left, fit);
+                    }
+                    if (bm_gains_pay(ctx, order, pass_accepts, left)) {
+                        bool ok = false;
+                        if ((s = bm_gains_build(ctx, &gains.g, &ok)) != BM_OK) return s;
+                        no_room = !ok;
+                        batch_s = 0;
+                    }
                 }
+                pass_t = secs_since(t0);
                 pass_full = true;
                 pass_accepts = 0;
             }

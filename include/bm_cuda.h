@@ -163,7 +163,7 @@ typedef struct bm_progress {
     int64_t evaluated;       /* exact deltas evaluated (full rows count n-1) */
     int64_t accepts;         /* swaps applied */
     int64_t score;           /* tracked score at return */
-    int64_t launches;        /* kernel batches launched */
+    int64_t launches;        /* batches evaluated; bm_search_batched counts those used, of which a launch may hold several */
     int32_t next_row_pos;    /* position in row_order to resume from */
     int32_t next_col;        /* column to resume from in that row */
     int32_t sweeps;          /* completed passes over row_order */
@@ -186,7 +186,9 @@ bm_status bm_sweep_parity(bm_ctx* ctx, const int32_t* row_order, int32_t nrows,
 /* Throughput search: batches of rows (row_order, cycled), best improving
  * partner per row, then a deterministic conflict-free subset of those swaps
  * (descending delta, ascending row) applied together.  Stops like
- * bm_sweep_parity; target_score > 0 also stops once the score reaches it. */
+ * bm_sweep_parity; target_score > 0 also stops once the score reaches it.
+ * While it runs it may hold two n x n tables of 32-bit gains, in at most half
+ * of the free device memory (see BM_PATH_GAIN_TABLES). */
 bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, int32_t nrows,
                             int32_t rows_per_batch, int64_t max_accepts, int32_t max_sweeps,
                             double time_budget_s, int64_t target_score, bm_progress* prog);
