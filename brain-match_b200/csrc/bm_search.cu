@@ -256,6 +256,11 @@ extern "C" bm_status bm_sweep_parity(bm_ctx* ctx, const int32_t* row_order, int3
     return ret;
 }
 
+// Rows of a launch of several batches at most: their staging is a megabyte of
+// pinned memory, whose pinning costs a context's first search milliseconds a
+// megabyte, and a launch of so many rows is far past where launches count.
+static constexpr int32_t kAheadRows = 20000;
+
 extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, int32_t nrows, int32_t rows_per_batch,
                                        int64_t max_accepts, int32_t max_sweeps, double time_budget_s,
                                        int64_t target_score, bm_progress* prog) {
@@ -269,8 +274,10 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
     const int32_t n = ctx->n;
     int32_t R = rows_per_batch > 0 ? rows_per_batch : 2 * ctx->num_sms;
     R = std::min(R, nr);
+    const int32_t most = std::min(nr, std::max(R, kAheadRows));  // rows of a launch
+    const int32_t max_ahead = most == nr ? (nr + R - 1) / R : most / R;
     SchedBufs b;
-    if ((s = sched_bufs(ctx, nr, &b)) != BM_OK) return s;
+    if ((s = sched_bufs(ctx, most, &b)) != BM_OK) return s;
     if ((s = bm_rows_refresh_work(ctx)) != BM_OK) return s;
     std::vector<int32_t> cand;
     BmMarks mk;
@@ -386,7 +393,7 @@ extern "C" bm_status bm_search_batched(bm_ctx* ctx, const int32_t* row_order, in
                 pass_accepts = 0;
             }
         }
-        ahead = na > 0 ? std::max(1, ahead / 2) : (int32_t)std::min<int64_t>(2 * (int64_t)ahead, (nr + R - 1) / R);
+        ahead = na > 0 ? std::max(1, ahead / 2) : std::min(2 * ahead, max_ahead);
     }
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     prog->next_row_pos = pos;
