@@ -423,44 +423,48 @@ struct GroupScratch {
 };
 
 // Whether k pairs, each u of which comes in runs of at least `run`, go to the
-// grouped kernel, with its scratch in place.  An item costs about 29 ns of the
-// chip (its tables, barriers and latency; full-scale pair), an entry of a pair
-// about 0.02 ns of the hash lookups' bandwidth: the grouped kernel pays when
-// its items, at most one per u, cost less than the pairs' entries.  Lists with
-// repeated neighbours have no dense table; the tables must fit in shared memory.
-bool use_groups(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t run) {
+// grouped kernel.  An item costs about 29 ns of the chip (its tables, barriers
+// and latency; full-scale pair), an entry of a pair about 0.02 ns of the hash
+// lookups' bandwidth: the grouped kernel pays when its items, at most one per
+// u, cost less than the pairs' entries.  Lists with repeated neighbours have no
+// dense table; the tables must fit in shared memory.
+bool groups_pay(const bm_ctx* ctx, int64_t k, int64_t run) {
     const int32_t mode = ctx->path[BM_PATH_PAIR_GROUPS];
-    if (mode < 0 || ctx->g[0].has_dup || ((uintptr_t)d_pairs & 7)) return false;
+    if (mode < 0 || ctx->g[0].has_dup) return false;
     if (group_smem(ctx->n) + 16384 > ctx->smem_optin) return false;
     const double items = (double)std::min<int64_t>(ctx->n, (k + run - 1) / run);
     const double entries = 2.0 * (double)(ctx->g[0].m_out + ctx->g[0].m_in) / ctx->n;  // of an average pair
-    if (mode == 0 && ((double)k * entries * 0.02 < 29.0 * items || k < 1024)) return false;
-    // the scratch is the context's: a capture's later replays would share it with
-    // whatever call comes then
+    return mode > 0 || ((double)k * entries * 0.02 >= 29.0 * items && k >= 1024);
+}
+
+size_t group_scratch(const bm_ctx* ctx, int64_t k) { return GroupScratch(ctx->n, std::min(k, kGrpChunk)).total; }
+
+// The context's own scratch for k pairs; null without room for it.
+void* context_scratch(bm_ctx* ctx, int64_t k) {
+    // a capture's later replays would share it with whatever call comes then
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-    const size_t need = GroupScratch(ctx->n, std::min(k, kGrpChunk)).total;
-    if (ctx->pscr_bytes >= need) return true;
+    if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
+    const size_t need = group_scratch(ctx, k);
+    if (ctx->pscr_bytes >= need) return ctx->pscr;
     // The call does not wait for the device: an outgrown block, which launches
     // in flight may use, is put by until the stream is next idle (bm_set_graph).
     // Blocks double up to the largest, so those put by hold about as much
     // together as the one in use at most.
-    const size_t most = GroupScratch(ctx->n, kGrpChunk).total, size = std::max(need, std::min(most, 2 * ctx->pscr_bytes));
+    const size_t size = std::max(need, std::min(group_scratch(ctx, kGrpChunk), 2 * ctx->pscr_bytes));
     void* block = nullptr;
     if (bm_cuda_malloc(&block, size) != cudaSuccess) {
         cudaGetLastError();  // no room for the sort: one warp per pair needs none
-        return false;
+        return nullptr;
     }
     if (ctx->pscr) ctx->pscr_old.push_back(ctx->pscr);
     ctx->pscr = block;
     ctx->pscr_bytes = size;
-    return true;
+    return block;
 }
 
-bm_status launch_groups(bm_ctx* ctx, const PairArgs& pa, const int32_t* d_pairs, int64_t k, int64_t* d_out) {
+bm_status launch_groups(bm_ctx* ctx, const PairArgs& pa, const int32_t* d_pairs, int64_t k, int64_t* d_out, char* base) {
     const int32_t n = ctx->n;
     const DevGraph &A = ctx->g[0], &B = ctx->g[1];
-    char* base = (char*)ctx->pscr;
     const GroupScratch L(n, std::min(k, kGrpChunk));
     // 1,024 threads when the tables leave room for one CTA on an SM, else as
     // many CTAs of 512 as fit: an item is a chain of short phases, which the
@@ -516,8 +520,8 @@ bm_status launch_groups(bm_ctx* ctx, const PairArgs& pa, const int32_t* d_pairs,
 
 }  // namespace
 
-bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_out, bool exact_only, int64_t run) {
-    if (k <= 0) return BM_OK;
+static bm_status launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_out, bool exact_only,
+                              void* scratch) {
     PairArgs a;
     a.A = gview(ctx->g[0]);
     a.selfB = ctx->g[1].self_w;
@@ -527,7 +531,7 @@ bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_
     a.n = ctx->n;
     a.refcpu = !exact_only && ctx->semantics == BM_SEMANTICS_REF_CPU;
     a.has_self = a.refcpu ? ctx->g[0].has_self : (ctx->g[0].has_self && ctx->g[1].has_self);
-    if (use_groups(ctx, d_pairs, k, std::max<int64_t>(1, run))) return launch_groups(ctx, a, d_pairs, k, d_out);
+    if (scratch) return launch_groups(ctx, a, d_pairs, k, d_out, (char*)scratch);
     // one pair to a block while the pairs are fewer than the resident blocks
     const int64_t slots = (int64_t)ctx->num_sms * 8;
     const int32_t per = (int32_t)std::max<int64_t>(1, std::min<int64_t>(kPairThreads / 32, k / slots));
@@ -535,6 +539,12 @@ bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_
     pairs_kernel<<<(unsigned)blocks, kPairThreads, 0, ctx->stream>>>(a, d_pairs, k, per, per == 1 ? 64 : 1024, d_out);
     BM_LAUNCH_CHECK(ctx, "pairs_kernel");
     return BM_OK;
+}
+
+bm_status bm_launch_pairs(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_out, bool exact_only, int64_t run) {
+    if (k <= 0) return BM_OK;
+    const bool grouped = ((uintptr_t)d_pairs & 7) == 0 && groups_pay(ctx, k, std::max<int64_t>(1, run));
+    return launch_pairs(ctx, d_pairs, k, d_out, exact_only, grouped ? context_scratch(ctx, k) : nullptr);
 }
 
 extern "C" bm_status bm_delta_pairs_dev(bm_ctx* ctx, const int32_t* d_pairs, int64_t k, int64_t* d_deltas) {
@@ -557,12 +567,21 @@ extern "C" bm_status bm_delta_pairs(bm_ctx* ctx, const int32_t* pairs, int64_t k
             return bm_fail(ctx, BM_INVALID_ARG, "pair entry %lld = %d outside 1..%d", (long long)i, pairs[i], ctx->n);
     const size_t in_bytes = sizeof(int32_t) * 2 * (size_t)k;
     const size_t in_al = (in_bytes + 255) & ~(size_t)255;
-    s = bm_stage(ctx, in_al + sizeof(int64_t) * (size_t)k);
+    // the sort's scratch is part of the call's staging: a context's first list
+    // grows its memory once
+    const size_t io = in_al + al256(sizeof(int64_t) * (size_t)k);
+    bool grouped = groups_pay(ctx, k, 1);
+    s = bm_stage(ctx, io + (grouped ? group_scratch(ctx, k) : 0));
+    if (s == BM_OOM && grouped) {
+        cudaGetLastError();
+        grouped = false;
+        s = bm_stage(ctx, io);
+    }
     if (s != BM_OK) return s;
     int32_t* d_pairs = (int32_t*)ctx->stage;
     int64_t* d_out = (int64_t*)((char*)ctx->stage + in_al);
     BM_CUDA(ctx, cudaMemcpyAsync(d_pairs, pairs, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
-    s = bm_launch_pairs(ctx, d_pairs, k, d_out);
+    s = launch_pairs(ctx, d_pairs, k, d_out, false, grouped ? (char*)ctx->stage + io : nullptr);
     if (s != BM_OK) return s;
     BM_CUDA(ctx, cudaMemcpyAsync(deltas, d_out, sizeof(int64_t) * (size_t)k, cudaMemcpyDeviceToHost, ctx->stream));
     BM_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
