@@ -559,9 +559,17 @@ extern "C" bm_status bm_delta_pairs(bm_ctx* ctx, const int32_t* pairs, int64_t k
     if (s != BM_OK) return s;
     if (k < 0 || (k > 0 && (!pairs || !deltas))) return bm_fail(ctx, BM_INVALID_ARG, "bad pair buffers");
     if (k == 0) return BM_OK;
+    // an id x in 1..n leaves the top bits of x - 1 and of n - x clear; sums of
+    // words, without comparisons or an early exit, are what the compiler turns into
+    // vectors (with a loop of comparisons a call of 2^20 pairs took 3.7 or 4.15 ms,
+    // by where the loop lay in the library; 3.4 ms so)
     const uint32_t un = (uint32_t)ctx->n;
-    bool bad = false;  // no early exit: the loop vectorises
-    for (int64_t i = 0; i < 2 * k; i++) bad |= (uint32_t)pairs[i] - 1u >= un;
+    uint32_t out_of_range = 0;
+    for (int64_t i = 0; i < 2 * k; i++) {
+        const uint32_t x = (uint32_t)pairs[i];
+        out_of_range |= (x - 1u) | (un - x);
+    }
+    const bool bad = out_of_range >> 31;
     for (int64_t i = 0; bad && i < 2 * k; i++)
         if (pairs[i] < 1 || pairs[i] > ctx->n)
             return bm_fail(ctx, BM_INVALID_ARG, "pair entry %lld = %d outside 1..%d", (long long)i, pairs[i], ctx->n);
