@@ -136,11 +136,11 @@ bm_status bm_launch_apply(bm_ctx* ctx, const int32_t* d_pairs, int32_t k) {
     a.pinv = ctx->pinv;
     a.ov = ctx->ov;
     a.ximg = ctx->ximg;
-    // blocks of a swap: one trip over the largest swap's lists (A's and B's
-    // largest degrees twice), while the swaps leave room for them.  The late
-    // launches of a full-scale search, whose swaps are hubs': 55 us in one
-    // block of 256 threads a swap, list by list, 11 us so; a swap of the
-    // 2,000-vertex pair 12.5 and 5.3 us
+    // blocks of a swap: about four entries a thread of the largest swap's lists
+    // (A's and B's largest degrees twice), up to 32 blocks and while the swaps
+    // leave room for them.  The late launches of a full-scale search, whose swaps
+    // are hubs': 55 us in one block of 256 threads a swap, list by list, 11 us so;
+    // a swap of the 2,000-vertex pair 12.5 and 5.3 us
     const int64_t most = 2 * ((int64_t)ctx->g[0].max_deg + B.max_deg);
     const unsigned parts = (unsigned)std::max<int64_t>(
         1, std::min<int64_t>({(most + 2 * kApplyThreads - 1) / (4 * kApplyThreads), (int64_t)ctx->num_sms * 8 / k, 32}));

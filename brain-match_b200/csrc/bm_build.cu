@@ -13,7 +13,8 @@
 // memory (36 MB at 3 M edges, about 4 ms) and of A's sorted lists back for the
 // host-side selection; the sorts move 8 bytes an edge and pass, eight passes.
 // Building the full-scale pair on the host took 190 ms for A and 390 ms for B;
-// it takes 8.6 and 12 ms so, the kernels 1.6 ms of them.
+// with each graph in one allocation (bm_graph_alloc) it takes 6.3-6.8 and 4.2-5.8
+// ms so, the kernels 1.6 ms of them.
 //
 // Inputs that the layout rejects (ids, weights, a second self-loop of an A
 // vertex, weighted degrees) only raise a flag here; the caller then has the

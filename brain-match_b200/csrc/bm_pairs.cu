@@ -77,7 +77,9 @@ __device__ __forceinline__ PairLists pair_lists(const PairArgs& a, int32_t u, in
 template <int STRIDE>
 __device__ __forceinline__ int32_t pair_share(const PairArgs& a, const PairLists& L, int32_t v, int32_t fu, int32_t fv,
                                               int t) {
-    int32_t s = 0;  // bounded by the weighted degrees of u and v, each below 2^29
+    // at most the weighted degrees of u and v for the terms and twice u's for the
+    // repair of its direct edges, each below 2^29: the pair's sum stays below 2^31
+    int32_t s = 0;
 #pragma unroll 2
     for (int32_t j = t; j < L.end.w; j += STRIDE) {
         const bool out = j < L.end.x || (j >= L.end.y && j < L.end.z);

@@ -24,7 +24,7 @@
 // few swaps, the gains of all rows are kept in tables (bm_gain.cu), so that a
 // batch is read instead of scattered.  The full-scale search from the greedy
 // start (60 passes, the last 50 with 146 accepts and fewer) took 735-755 ms with
-// one scattered batch a launch and takes 300-330 ms so.
+// one scattered batch a launch and takes 290-345 ms so, by the box.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
