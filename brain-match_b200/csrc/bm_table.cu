@@ -94,21 +94,30 @@ __device__ __forceinline__ PairRows block_pairs(int32_t n) {
     return r;
 }
 
-// Visit the upper triangle of this block's rows with 16-byte streaming loads
-// (rows start 16-byte aligned: ld is a multiple of 4).  The group loop is
+// Four entries of a row, columns v .. v + 3: one 16-byte streaming load, or, where
+// rows are not on 16-byte boundaries, the entries up to column n one by one.
+__device__ __forceinline__ int4 load_group(const int32_t* __restrict__ row, int32_t v, int32_t n, bool vec) {
+    if (vec) return __ldcs(reinterpret_cast<const int4*>(row + v));
+    return make_int4(v <= n ? row[v] : 0, v + 1 <= n ? row[v + 1] : 0, v + 2 <= n ? row[v + 2] : 0,
+                     v + 3 <= n ? row[v + 3] : 0);
+}
+
+// Visit the upper triangle of this block's rows, four entries a thread at a
+// time; the array may start anywhere and have any stride.  The group loop is
 // uniform over the block; f(u, v, d, ok) sees every lane, ok marks v in (u, n].
 // Any order: used by the passes that do not depend on it.
 template <class F>
 __device__ __forceinline__ void scan_upper(const int32_t* __restrict__ tab, int64_t ld, int32_t n, F&& f) {
+    const bool vec = (ld & 3) == 0 && ((uintptr_t)tab & 15) == 0;
     const PairRows pr = block_pairs(n);
     for (int32_t j = 0; j < pr.rows(); j++) {
         const int32_t u = pr.row(j);
-        const int4* r4 = reinterpret_cast<const int4*>(tab + (size_t)u * (size_t)ld);
+        const int32_t* row = tab + (size_t)u * (size_t)ld;
         const int32_t g0 = (u + 1) >> 2, g1 = n >> 2;
         for (int32_t gb = g0; gb <= g1; gb += 2 * kTabThreads) {
             const int32_t ga = gb + (int32_t)threadIdx.x, gc = ga + kTabThreads;
-            const int4 qa = ga <= g1 ? __ldcs(r4 + ga) : make_int4(0, 0, 0, 0);
-            const int4 qc = gc <= g1 ? __ldcs(r4 + gc) : make_int4(0, 0, 0, 0);
+            const int4 qa = ga <= g1 ? load_group(row, 4 * ga, n, vec) : make_int4(0, 0, 0, 0);
+            const int4 qc = gc <= g1 ? load_group(row, 4 * gc, n, vec) : make_int4(0, 0, 0, 0);
             const int32_t da[4] = {qa.x, qa.y, qa.z, qa.w}, dc[4] = {qc.x, qc.y, qc.z, qc.w};
 #pragma unroll
             for (int c = 0; c < 4; c++) {
