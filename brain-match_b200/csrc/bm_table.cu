@@ -94,21 +94,26 @@ __device__ __forceinline__ PairRows block_pairs(int32_t n) {
     return r;
 }
 
-// Four entries of a row, columns v .. v + 3: one 16-byte streaming load, or, where
-// rows are not on 16-byte boundaries, the entries up to column n one by one.
-__device__ __forceinline__ int4 load_group(const int32_t* __restrict__ row, int32_t v, int32_t n, bool vec) {
-    if (vec) return __ldcs(reinterpret_cast<const int4*>(row + v));
-    return make_int4(v <= n ? row[v] : 0, v + 1 <= n ? row[v + 1] : 0, v + 2 <= n ? row[v + 2] : 0,
-                     v + 3 <= n ? row[v + 3] : 0);
+// Group g of a row, columns 4 g .. 4 g + 3: one 16-byte streaming load, or, where
+// rows are not on 16-byte boundaries (VEC false), the entries up to column n one
+// by one.
+template <bool VEC>
+__device__ __forceinline__ int4 load_group(const int32_t* __restrict__ row, int32_t g, int32_t n) {
+    if constexpr (VEC) {
+        return __ldcs(reinterpret_cast<const int4*>(row) + g);
+    } else {
+        const int32_t v = 4 * g;
+        return make_int4(v <= n ? row[v] : 0, v + 1 <= n ? row[v + 1] : 0, v + 2 <= n ? row[v + 2] : 0,
+                         v + 3 <= n ? row[v + 3] : 0);
+    }
 }
 
 // Visit the upper triangle of this block's rows, four entries a thread at a
 // time; the array may start anywhere and have any stride.  The group loop is
 // uniform over the block; f(u, v, d, ok) sees every lane, ok marks v in (u, n].
 // Any order: used by the passes that do not depend on it.
-template <class F>
+template <bool VEC, class F>
 __device__ __forceinline__ void scan_upper(const int32_t* __restrict__ tab, int64_t ld, int32_t n, F&& f) {
-    const bool vec = (ld & 3) == 0 && ((uintptr_t)tab & 15) == 0;
     const PairRows pr = block_pairs(n);
     for (int32_t j = 0; j < pr.rows(); j++) {
         const int32_t u = pr.row(j);
@@ -116,8 +121,8 @@ __device__ __forceinline__ void scan_upper(const int32_t* __restrict__ tab, int6
         const int32_t g0 = (u + 1) >> 2, g1 = n >> 2;
         for (int32_t gb = g0; gb <= g1; gb += 2 * kTabThreads) {
             const int32_t ga = gb + (int32_t)threadIdx.x, gc = ga + kTabThreads;
-            const int4 qa = ga <= g1 ? load_group(row, 4 * ga, n, vec) : make_int4(0, 0, 0, 0);
-            const int4 qc = gc <= g1 ? load_group(row, 4 * gc, n, vec) : make_int4(0, 0, 0, 0);
+            const int4 qa = ga <= g1 ? load_group<VEC>(row, ga, n) : make_int4(0, 0, 0, 0);
+            const int4 qc = gc <= g1 ? load_group<VEC>(row, gc, n) : make_int4(0, 0, 0, 0);
             const int32_t da[4] = {qa.x, qa.y, qa.z, qa.w}, dc[4] = {qc.x, qc.y, qc.z, qc.w};
 #pragma unroll
             for (int c = 0; c < 4; c++) {
@@ -136,6 +141,7 @@ __device__ __forceinline__ void scan_upper(const int32_t* __restrict__ tab, int6
 // Histogram of one digit over the entries whose fixed digits match.  Deltas
 // crowd into a few bins, so each thread merges runs of equal bins in a
 // register and adds a run with one shared-memory atomic.
+template <bool VEC>
 __global__ void __launch_bounds__(kTabThreads) hist_kernel(const int32_t* __restrict__ tab, int64_t ld, int32_t n,
                                                            const TopState* st, int shift, int bits,
                                                            uint32_t* __restrict__ ghist) {
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(kTabThreads) hist_kernel(const int32_t* __rest
     __syncthreads();
     const uint32_t prefix = st->prefix, mask = st->mask, dm = (1u << bits) - 1u;
     uint32_t run_bin = 0, run_cnt = 0;
-    scan_upper(tab, ld, n, [&](int32_t, int32_t, int32_t d, bool ok) {
+    scan_upper<VEC>(tab, ld, n, [&](int32_t, int32_t, int32_t d, bool ok) {
         const uint32_t key = okey(d);
         if (ok && (key & mask) == prefix) {
             const uint32_t b = (key >> shift) & dm;
@@ -217,12 +223,13 @@ struct Sel {
 // ties per block.
 // Entries above the threshold (any order, atomic slots), and the ties per
 // row (each thread adds its count for a row when it moves to another row).
+template <bool VEC>
 __global__ void __launch_bounds__(kTabThreads) gather_gt_kernel(const int32_t* __restrict__ tab, int64_t ld, int32_t n,
                                                                 TopState* st, Sel sel, int32_t* __restrict__ rowtie) {
     const uint32_t T = st->prefix;
     const int32_t n_gt = st->k - st->need;
     int32_t cur = 0, eq = 0;
-    scan_upper(tab, ld, n, [&](int32_t u, int32_t v, int32_t d, bool ok) {
+    scan_upper<VEC>(tab, ld, n, [&](int32_t u, int32_t v, int32_t d, bool ok) {
         const uint32_t key = okey(d);
         if (ok && key > T) {
             const int32_t slot = atomicAdd(&st->gt_slot, 1);
@@ -519,16 +526,19 @@ static bm_status bm_table_topk_launch(bm_ctx* ctx, const int32_t* d_tab, int64_t
     TopState h{0u, 0u, keff, 0, keff, 0};
     BM_CUDA(ctx, cudaMemcpyAsync(S.st, &h, sizeof(TopState), cudaMemcpyHostToDevice, ctx->stream));
     BM_CUDA(ctx, cudaMemsetAsync(S.hist, 0, sizeof(uint32_t) * kBins, ctx->stream));
+    const bool vec = (ld & 3) == 0 && ((uintptr_t)d_tab & 15) == 0;
     if (keff > 0) {
         const int shifts[3] = {21, 10, 0}, widths[3] = {11, 11, 10};
         for (int p = 0; p < 3; p++) {
-            hist_kernel<<<kTabBlocks, kTabThreads, 0, ctx->stream>>>(d_tab, ld, n, S.st, shifts[p], widths[p], S.hist);
+            (vec ? hist_kernel<true> : hist_kernel<false>)<<<kTabBlocks, kTabThreads, 0, ctx->stream>>>(
+                d_tab, ld, n, S.st, shifts[p], widths[p], S.hist);
             BM_LAUNCH_CHECK(ctx, "hist_kernel");
             select_digit_kernel<<<1, kSelThreads, 0, ctx->stream>>>(S.hist, S.st, shifts[p], widths[p]);
             BM_LAUNCH_CHECK(ctx, "select_digit_kernel");
         }
         BM_CUDA(ctx, cudaMemsetAsync(S.rowtie, 0, sizeof(int32_t) * ((size_t)n + 2), ctx->stream));
-        gather_gt_kernel<<<kTabBlocks, kTabThreads, 0, ctx->stream>>>(d_tab, ld, n, S.st, S.sel, S.rowtie);
+        (vec ? gather_gt_kernel<true> : gather_gt_kernel<false>)<<<kTabBlocks, kTabThreads, 0, ctx->stream>>>(
+            d_tab, ld, n, S.st, S.sel, S.rowtie);
         BM_LAUNCH_CHECK(ctx, "gather_gt_kernel");
         scan_rows_kernel<<<1, kScanThreads, 0, ctx->stream>>>(S.rowtie, n + 2);
         BM_LAUNCH_CHECK(ctx, "scan_rows_kernel");
